@@ -319,7 +319,7 @@ void free_ctx(z4c_ctx* c) {
   c->reg[Z4C_REG_TAN] = c->reg[Z4C_REG_ADJ] = c->reg[Z4C_REG_ADM_ADJ] = nullptr;
   for (auto& r : c->reg)
     if (r) cudaFree(r);
-  for (void* p : {(void*)c->un, (void*)c->guu, (void*)c->sd, (void*)c->rsum, (void*)c->lv, (void*)c->xf, (void*)c->xv, (void*)c->dxd, (void*)c->fd,
+  for (void* p : {(void*)c->un, (void*)c->guu, (void*)c->sd, (void*)c->xf, (void*)c->xv, (void*)c->dxd, (void*)c->fd,
                   (void*)c->nbr, (void*)c->partials, (void*)c->flag, (void*)c->trk})
     if (p) cudaFree(p);
   for (auto& w : c->waves) wave_free(&w);
@@ -553,12 +553,21 @@ int create_impl(const z4c_mesh_desc_t* mesh, const z4c_params_t* params, int int
   }
   if (rc == Z4C_OK && integrator == Z4C_INTEG_BT_RK4) rc = alloc((void**)&c->un, b22);
   if (rc == Z4C_OK) rc = alloc((void**)&c->guu, sizeof(double) * 6 * (size_t)g.nvol * nb);
-  if (rc == Z4C_OK)
-    rc = alloc((void**)&c->sd, sizeof(double) * kSdComponents * (size_t)g.nvol * nb);
-  if (rc == Z4C_OK)
-    rc = alloc((void**)&c->rsum, sizeof(double) * 6 * (size_t)interior_count(g) * nb);
-  if (rc == Z4C_OK)
-    rc = alloc((void**)&c->lv, sizeof(double) * Z4C_NVAR * (size_t)interior_count(g) * nb);
+  {
+    // The right-hand-side scratch: the diagnostics' and the adjoint's three
+    // arrays, or the derivative pass's components of every interior vertex
+    // where that is at most a little more or small in itself (otherwise the
+    // passes run in pieces that fit).
+    const int64_t npts = interior_count(g), first = (int64_t)kSdComponents * g.nvol * nb;
+    const int64_t parts = first + 28 * npts * nb, whole = rhs_scratch_doubles(g) * nb;
+    c->scratch_cap = whole <= parts + parts / 16 || whole <= (int64_t)1 << 29
+                         ? std::max(parts, whole) : parts;
+    if (rc == Z4C_OK) rc = alloc((void**)&c->sd, sizeof(double) * (size_t)c->scratch_cap);
+    if (rc == Z4C_OK) {
+      c->rsum = c->sd + first;
+      c->lv = c->rsum + 6 * npts * nb;
+    }
+  }
   if (rc == Z4C_OK) rc = alloc((void**)&c->xf, sizeof(double) * c->h_xf.size());
   if (rc == Z4C_OK) rc = alloc((void**)&c->xv, sizeof(double) * c->h_xv.size());
   if (rc == Z4C_OK) rc = alloc((void**)&c->dxd, sizeof(double) * c->h_dx.size());
@@ -1157,24 +1166,10 @@ int z4c_autotune(z4c_ctx* ctx, int reps, float* best_ms_out) {
   if (ctx->integrator != Z4C_INTEG_RK4)
     return fail(Z4C_ESTATE, "the autotuner times the low-storage stage");
   if (reps < 1) reps = 1;
-  // greedy: the heavy passes' CTA size first, then the column passes' shape;
   // the stage writes only the work register, u1 and rhs, so u is untouched
   LaunchShape best = ctx->shape;
   float best_ms = 1e30f, ms = 0.f;
   int rc;
-  for (int pt : {64, 128, 256})
-    for (int regs : {0, kPointRegsHigh}) {
-      if (regs && (pt == 256 || !has_fixed_geometry(ctx->g))) continue;
-      LaunchShape sh = best;
-      sh.point_threads = pt;
-      sh.point_regs = regs;
-      if ((rc = time_stage(ctx, sh, reps, &ms))) return rc;
-      if (ms < best_ms) {
-        best_ms = ms;
-        best.point_threads = pt;
-        best.point_regs = regs;
-      }
-    }
   for (int ct : {128, 256, 512})
     for (int ns : {0, 1, 2, 3, 4}) {
       LaunchShape sh = best;

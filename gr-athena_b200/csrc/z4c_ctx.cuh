@@ -62,9 +62,11 @@ struct z4c_ctx {
   double* reg[Z4C_NREG] = {};
   double* un = nullptr;   // Butcher u_n scratch
   double* guu = nullptr;  // ADMToZ4c inverse-metric scratch (6 vars)
-  double* sd = nullptr;   // stored first derivatives, 33 values per vertex
-  double* rsum = nullptr; // Ricci-pass scratch, 6 values per interior vertex
-  double* lv = nullptr;   // advection sums, 22 values per interior vertex
+  double* sd = nullptr;   // right-hand-side scratch; its parts when used as such:
+                          // stored first derivatives, 33 values per vertex,
+  double* rsum = nullptr; // then Ricci sums, 6 values per interior vertex,
+  double* lv = nullptr;   // then 22 values per interior vertex
+  int64_t scratch_cap = 0;  // doubles at sd
   double* xf = nullptr;   // [nblocks][nn0+nn1+nn2]
   double* xv = nullptr;   // [nblocks][nn0+nn1+nn2-3]
   double* dxd = nullptr;  // [nblocks][3] vertex spacing
@@ -98,7 +100,7 @@ struct z4c_ctx {
   double graph_dt = 0.0;
   bool graph_per_block = false;
 
-  RhsScratch scratch() const { return RhsScratch{sd, rsum, lv}; }
+  RhsScratch scratch() const { return RhsScratch{sd, rsum, lv, sd, scratch_cap}; }
 
   DevParams dev() const {
     DevParams P;

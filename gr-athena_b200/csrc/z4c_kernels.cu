@@ -16,21 +16,12 @@ namespace z4c {
 
 namespace {
 
-// Launch shapes.  The heavy per-vertex passes (k_ricci, k_main) are compiled
-// for 64, 128 and 256 threads per CTA (all at the full register file of
-// 255 registers per thread); the column passes for k-loop unrolls of 2 and 4
-// and up to 512 threads per CTA.  A context's shape comes from the
-// autotuner (z4c_autotune) or from z4c_set_tile.
+// Launch shapes.  The column passes take up to 512 threads per CTA; a
+// context's shape comes from the autotuner (z4c_autotune) or z4c_set_tile.
 constexpr int kPointThreads = 256;
 constexpr int kColumnMaxThreads = 512;
 
 inline int div_up(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
-
-// Rsum scratch: [block][6][interior vertex], interior vertices in i-fastest
-// order.
-__device__ __forceinline__ double* rsum_at(const Grid& g, double* rsum, int b, int64_t l) {
-  return rsum + (int64_t)b * 6 * interior_count(g) + l;
-}
 
 // ---- stored first derivatives (Z4c::PrepareZ4cDerivatives) ----------------
 // adm_z4c.cpp:972-1037: D_b f for f in chi, g~_ab, alpha, beta^a.  The
@@ -95,22 +86,22 @@ k_prep(Grid gin, DevParams P, const double* __restrict__ u, double* __restrict__
 template <int THREADS, int NX, int MINB = 1>
 __global__ void __launch_bounds__(THREADS, MINB)
 k_ricci(Grid gin, DevParams P, const double* __restrict__ u, const double* __restrict__ sd,
-        double* __restrict__ rsum, int block0, int nblk) {
+        double* __restrict__ rsum, int block0) {
   const Grid g = fixed_geometry<NX>(gin);
-  const int64_t npts = interior_count(g);
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= npts * nblk) return;
-  const int b = block0 + (int)(t / npts);
-  const int64_t l = t % npts;
+  const int npts = (int)interior_count(g);
+  const int l = (int)(blockIdx.x * THREADS + threadIdx.x);
+  if (l >= npts) return;
+  const int b = block0 + (int)blockIdx.y;
   int i, j, k;
   interior_ijk(g, l, i, j, k);
-  const int64_t p = ((int64_t)k * g.nn[1] + j) * g.nn[0] + i;
-  double R[6];
-  ricci_point(u + (int64_t)b * NVAR * g.nvol, sd + (int64_t)b * kSdComponents * g.nvol, g.nvol,
-              p, g.s, P, P.fd[b], R);
-  double* rs = rsum_at(g, rsum, b, l);
+  const unsigned pb = 8u * (unsigned)((k * g.nn[1] + j) * g.nn[0] + i), lb = 8u * (unsigned)l;
+  const StencilSrc src{u + (int64_t)b * NVAR * g.nvol, sd + (int64_t)b * kSdComponents * g.nvol,
+                       g.nvol, g.s, &P.fd[b], pb};
+  double g_dd[6], g_uu[6], Gamma_udd[3][6], Gamma_u[3], R[6];
+  ricci_point(src, P.p, g_dd, g_uu, Gamma_udd, Gamma_u, R);
+  double* rs = rsum + (int64_t)b * 6 * npts;
 #pragma unroll
-  for (int q = 0; q < 6; ++q) rs[(int64_t)q * npts] = R[q];
+  for (int q = 0; q < 6; ++q) sto(rs + (int64_t)q * npts, lb, R[q]);
 }
 
 
@@ -192,55 +183,23 @@ k_sommerfeld(Grid g, DevParams P, const double* __restrict__ u, double* __restri
   rhs[q] = sommerfeld_value(g, P, b, n, u + q, i, j, k, g.s);
 }
 
-// Advection sums (calculate_z4c_rhs.cpp:184-226): lv [block][22][interior vertex]
-template <int UNROLL, int NX>
-__global__ void __launch_bounds__(kColumnMaxThreads)
-k_adv(Grid gin, DevParams P, const double* __restrict__ u, double* __restrict__ lv, int block0,
-      int nblk) {
-  const Grid g = fixed_geometry<NX>(gin);
-  Column c;
-  if (!column_index(g, block0, nblk, c)) return;
-  const int nn0 = g.nn[0], sk = nn0 * g.nn[1];
-  const int n0 = g.nx[0] + 1, n1 = g.nx[1] + 1;
-  const int64_t npts = interior_count(g);
-  const double* U = u + (int64_t)c.b * NVAR * g.nvol + c.j * nn0 + c.i;
-  const double* f = U + (int64_t)c.n * g.nvol;
-  const double* bx = U + (int64_t)Z4C_BETAX * g.nvol;
-  const double* by = U + (int64_t)Z4C_BETAY * g.nvol;
-  const double* bz = U + (int64_t)Z4C_BETAZ * g.nvol;
-  double* out = lv + ((int64_t)c.b * NVAR + c.n) * npts + (c.j - NG) * n0 + (c.i - NG);
-  const FdScale& F = P.fd[c.b];
-  double w[9];
-  window_init(f, sk, NG, w);
-#pragma unroll UNROLL
-  for (int k = NG; k <= NG + g.nx[2]; ++k) {
-    window_advance(f, sk, k, w);
-    const int o = k * sk;
-    double acc = 0;
-    acc += fd_lx_side(f + o, 1, __ldg(bx + o), F.lidx[0]);
-    acc += fd_lx_side(f + o, nn0, __ldg(by + o), F.lidx[1]);
-    acc += fd_lx_window(w, __ldg(bz + o), F.lidx[2]);
-    out[(k - NG) * n0 * n1] = acc;
-    window_shift(w);
-  }
-}
-
 // Z4cRHS tail: rhs += KO, in place.
-template <int UNROLL, int NX>
+template <int UNROLL, bool WHOLE, int NX>
 __global__ void __launch_bounds__(kColumnMaxThreads)
 k_ko_rhs(Grid gin, DevParams P, const double* __restrict__ u, double* __restrict__ rhs,
-         int block0, int nblk) {
+         int block0,
+      int nblk, ColChunks T) {
   const Grid g = fixed_geometry<NX>(gin);
   Column c;
-  if (!column_index(g, block0, nblk, c)) return;
+  if (!column_index<WHOLE>(g, T, block0, nblk, c)) return;
   const int nn0 = g.nn[0], sk = nn0 * g.nn[1];
   const int64_t base = ((int64_t)c.b * NVAR + c.n) * g.nvol + c.j * nn0 + c.i;
   const double* f = u + base;
   const FdScale& F = P.fd[c.b];
   double w[9];
-  window_init(f, sk, NG, w);
+  window_init(f, sk, c.k0, w);
 #pragma unroll UNROLL
-  for (int k = NG; k <= NG + g.nx[2]; ++k) {
+  for (int k = c.k0; k <= c.k1; ++k) {
     window_advance(f, sk, k, w);
     const int o = k * sk;
     rhs[base + o] = add_ko_column(rhs[base + o], f + o, nn0, w, F, P.p.diss);
@@ -255,14 +214,15 @@ k_ko_rhs(Grid gin, DevParams P, const double* __restrict__ u, double* __restrict
 //   WeightedAve(u1, u, u2, {1, delta, 0}); WeightedAve(u, u1, u2, {g1, g2, g3});
 //   AddZ4cRHS(rhs, beta*dt, u)        (mesh/weighted_ave.cpp:20-150)
 // u is read (all points, for the stencils); u_out, u1 are written (interior).
-template <int UNROLL, bool SOM, int NX>
+template <int UNROLL, bool WHOLE, bool SOM, int NX>
 __global__ void __launch_bounds__(kColumnMaxThreads)
 k_ko_stage_ls(Grid gin, DevParams P, const double* __restrict__ u,
               const double* __restrict__ rhs, double* __restrict__ u1,
-              double* __restrict__ u_out, LsStage w, int block0, int nblk) {
+              double* __restrict__ u_out, LsStage w, int block0,
+      int nblk, ColChunks T) {
   const Grid g = fixed_geometry<NX>(gin);
   Column c;
-  if (!column_index(g, block0, nblk, c)) return;
+  if (!column_index<WHOLE>(g, T, block0, nblk, c)) return;
   const int nn0 = g.nn[0], sk = nn0 * g.nn[1];
   const int64_t base = ((int64_t)c.b * NVAR + c.n) * g.nvol + c.j * nn0 + c.i;
   const double* f = u + base;
@@ -270,9 +230,9 @@ k_ko_stage_ls(Grid gin, DevParams P, const double* __restrict__ u,
   // Z4cBoundaryRHS replaces this variable's right-hand side on Sommerfeld faces
   const bool som = SOM && sommerfeld_var(c.n);
   double win[9];
-  window_init(f, sk, NG, win);
+  window_init(f, sk, c.k0, win);
 #pragma unroll UNROLL
-  for (int k = NG; k <= NG + g.nx[2]; ++k) {
+  for (int k = c.k0; k <= c.k1; ++k) {
     window_advance(f, sk, k, win);
     const int o = k * sk;
     const int64_t q = base + o;
@@ -292,14 +252,15 @@ k_ko_stage_ls(Grid gin, DevParams P, const double* __restrict__ u,
 struct KPtrs {
   double* k[4];
 };
-template <int UNROLL, bool SOM, int NX>
+template <int UNROLL, bool WHOLE, bool SOM, int NX>
 __global__ void __launch_bounds__(kColumnMaxThreads)
 k_ko_stage_bt(Grid gin, DevParams P, const double* __restrict__ u, const double* __restrict__ rhs,
               const double* __restrict__ un, KPtrs K, double* __restrict__ u_out, BtStage w,
-              int block0, int nblk) {
+              int block0,
+      int nblk, ColChunks T) {
   const Grid g = fixed_geometry<NX>(gin);
   Column c;
-  if (!column_index(g, block0, nblk, c)) return;
+  if (!column_index<WHOLE>(g, T, block0, nblk, c)) return;
   const int nn0 = g.nn[0], sk = nn0 * g.nn[1];
   const int64_t base = ((int64_t)c.b * NVAR + c.n) * g.nvol + c.j * nn0 + c.i;
   const double* f = u + base;
@@ -307,9 +268,9 @@ k_ko_stage_bt(Grid gin, DevParams P, const double* __restrict__ u, const double*
   // Z4cBoundaryRHS replaces this variable's right-hand side on Sommerfeld faces
   const bool som = SOM && sommerfeld_var(c.n);
   double win[9];
-  window_init(f, sk, NG, win);
+  window_init(f, sk, c.k0, win);
 #pragma unroll UNROLL
-  for (int k = NG; k <= NG + g.nx[2]; ++k) {
+  for (int k = c.k0; k <= c.k1; ++k) {
     window_advance(f, sk, k, win);
     const int o = k * sk;
     const int64_t q = base + o;
@@ -359,57 +320,6 @@ __device__ __forceinline__ void slab_load(double* __restrict__ sm, const double*
   }
   asm volatile("cp.async.wait_all;\n" ::: "memory");
   __syncthreads();
-}
-
-// Advection sums, and for chi, g~, alpha, beta the stored first derivatives
-// (the work of k_adv and k_prep on one variable).
-__global__ void __launch_bounds__(kColumnMaxThreads)
-k_adv_prep_slab(Grid g, DevParams P, const double* __restrict__ u, double* __restrict__ lv,
-                double* __restrict__ sd, SlabGeom S, int block0) {
-  extern __shared__ double sm[];
-  const int n = (int)blockIdx.y, b = block0 + (int)blockIdx.z;
-  int kl, kh;
-  slab_range(g, S, kl, kh);
-  if (kl > kh) return;
-  const int nn0 = g.nn[0], pl = S.plane;
-  const double* U = u + (int64_t)b * NVAR * g.nvol;
-  slab_load(sm, U + (int64_t)n * g.nvol, kl, kh, pl);
-  // vertex (i, j, k) of the block in shared memory
-  const double* s0 = sm - (int64_t)(kl - NG) * pl;
-  const FdScale& F = P.fd[b];
-  const int n0 = g.nx[0] + 1, n1 = g.nx[1] + 1, nk = kh - kl + 1;
-  const int64_t npts = interior_count(g);
-  double* out = lv + ((int64_t)b * NVAR + n) * npts;
-  for (int q = threadIdx.x; q < n0 * n1 * nk; q += blockDim.x) {
-    const int i = NG + q % n0, j = NG + (q / n0) % n1, k = kl + q / (n0 * n1);
-    const int o = k * pl + j * nn0 + i;
-    double acc = 0;
-    acc += fd_lx_side<false>(s0 + o, 1, __ldg(U + (int64_t)Z4C_BETAX * g.nvol + o), F.lidx[0]);
-    acc += fd_lx_side<false>(s0 + o, nn0, __ldg(U + (int64_t)Z4C_BETAY * g.nvol + o), F.lidx[1]);
-    acc += fd_lx_side<false>(s0 + o, pl, __ldg(U + (int64_t)Z4C_BETAZ * g.nvol + o), F.lidx[2]);
-    out[((k - NG) * n1 + (j - NG)) * n0 + (i - NG)] = acc;
-  }
-  // stored first derivatives (k_prep's regions): D_x on the interior, D_y
-  // extended by 3 along x, D_z extended by 3 along x and y
-  int slot = -1;
-#pragma unroll
-  for (int q = 0; q < kSdFields; ++q)
-    if (sd_field_var(q) == n) slot = q;
-  if (slot < 0) return;
-  double* sdb = sd + ((int64_t)b * kSdComponents + slot * 3) * g.nvol;
-  for (int dir = 0; dir < 3; ++dir) {
-    const int ex = (dir >= 1) ? 3 : 0, ey = (dir == 2) ? 3 : 0;
-    const int e0 = n0 + 2 * ex, e1 = n1 + 2 * ey;
-    const int st = (dir == 0) ? 1 : (dir == 1 ? nn0 : pl);
-    const double c1 = F.cidx1[dir];
-    double* o_dir = sdb + (int64_t)dir * g.nvol;
-    for (int q = threadIdx.x; q < e0 * e1 * nk; q += blockDim.x) {
-      const int i = NG - ex + q % e0, j = NG - ey + (q / e0) % e1, k = kl + q / (e0 * e1);
-      const int o = k * pl + j * nn0 + i;
-      const double* v = s0 + o;
-      o_dir[o] = fd_dx7(v[-3 * st], v[-2 * st], v[-st], v[st], v[2 * st], v[3 * st], c1);
-    }
-  }
 }
 
 // Kreiss-Oliger from shared memory, rhs += Diss_x; += Diss_y; += Diss_z.
@@ -517,28 +427,29 @@ k_ko_rhs_slab(Grid g, DevParams P, const double* __restrict__ u, double* __restr
   }
 }
 
-// ---- main pass: the right-hand side without the Kreiss-Oliger terms -------
-template <int THREADS, int NX, int MINB = 1>
-__global__ void __launch_bounds__(THREADS, MINB)
-k_main(Grid gin, DevParams P, const double* __restrict__ u, const double* __restrict__ sd,
-       const double* __restrict__ rsum, const double* __restrict__ lv, double* __restrict__ rhs,
-       int block0, int nblk) {
-  const Grid g = fixed_geometry<NX>(gin);
-  const int64_t npts = interior_count(g);
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= npts * nblk) return;
-  const int b = block0 + (int)(t / npts);
-  const int64_t l = t % npts;
-  int i, j, k;
-  interior_ijk(g, l, i, j, k);
+// ---- pointwise pass: the right-hand side without the Kreiss-Oliger terms ----
+// One warp per 32 interior vertices, their operands staged in shared memory
+// (stage_group); five warps per SM keep 200 kB in flight.  Bound by DRAM: 512
+// blocks of 16^3, 0.78 ms, 4.1 GB (5.2 TB/s); with the operands loaded where
+// they are used, at eight warps per SM, 0.98 ms.
+__global__ void __launch_bounds__(kDvGroup)
+k_point(Grid g, DevParams P, const double* __restrict__ u, const double* __restrict__ D,
+        double* __restrict__ rhs, int block0, int ks, int nk) {
+  extern __shared__ double sm[];
+  const int n0 = g.nx[0] + 1, n1 = g.nx[1] + 1, np = nk * n1 * n0;
+  const int l = (int)(blockIdx.x * kDvGroup + threadIdx.x);
+  const int64_t b = block0 + (int)blockIdx.y;
+  const int i = NG + l % n0, j = NG + (l / n0) % n1, k = NG + ks + l / (n0 * n1);
+  const int64_t at = b * NVAR * g.nvol;
   const int64_t p = ((int64_t)k * g.nn[1] + j) * g.nn[0] + i;
+  const DerivSrc src = stage_group(
+      sm, D + blockIdx.y * dv_doubles(np) + (int64_t)blockIdx.x * (kDvComponents * kDvGroup),
+      u + at + p, g.nvol, l < np);
+  if (l >= np) return;
   double out[NVAR];
-  rhs_point(u + (int64_t)b * NVAR * g.nvol, sd + (int64_t)b * kSdComponents * g.nvol, g.nvol, p,
-            g.s, P, P.fd[b], rsum + (int64_t)b * 6 * npts + l, lv + (int64_t)b * NVAR * npts + l,
-            npts, out);
-  double* rb = rhs + (int64_t)b * NVAR * g.nvol + p;
+  rhs_point<true>(src, P.p, out);
 #pragma unroll
-  for (int n = 0; n < NVAR; ++n) rb[(int64_t)n * g.nvol] = out[n];
+  for (int n = 0; n < NVAR; ++n) rhs[at + n * g.nvol + p] = out[n];
 }
 
 // ---- puncture tracker (z4c/puncture_tracker.cpp) ----------------------------
@@ -1268,15 +1179,6 @@ long long kernel_launch_count() { return g_launches.load(); }
 void add_kernel_launches(long long n) { g_launches += n; }
 #define COUNTED ++g_launches;
 
-// Unroll of the column passes' z loops (loads in flight per thread): the
-// fixed-geometry instances unroll their nx + 1 iterations completely, the
-// generic ones by kColUnroll.
-constexpr int kColUnroll = 4;
-
-// Threads of the column passes (one per block, variable and interior (i, j)).
-static int64_t columns(const Grid& g, int nblk) {
-  return (int64_t)(g.nx[0] + 1) * (g.nx[1] + 1) * NVAR * nblk;
-}
 
 bool valid_shape(const LaunchShape& sh) {
   return (sh.point_regs == 0 || sh.point_regs == kPointRegsHigh) &&
@@ -1285,6 +1187,11 @@ bool valid_shape(const LaunchShape& sh) {
           sh.column_threads == 512) &&
          (sh.column_slabs >= 0 && sh.column_slabs <= 4);
 }
+
+// Unroll of the column passes' z loops (loads in flight per thread): the
+// fixed-geometry instances unroll their nx + 1 iterations completely, the
+// generic ones by kColUnroll.
+constexpr int kColUnroll = 4;
 
 // Shared-memory slab geometry of a shape, or kper = 0 when the per-variable
 // passes run as pencils (column_slabs = 0, or planes that do not fit).
@@ -1315,80 +1222,71 @@ int allow_slab_smem() {
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSlabMaxBytes);
     if (e == cudaSuccess) e = r;
   };
-  set((const void*)k_adv_prep_slab);
   set((const void*)k_ko_rhs_slab);
   set((const void*)k_ko_stage_ls_slab<true>);
   set((const void*)k_ko_stage_ls_slab<false>);
   set((const void*)k_ko_stage_bt_slab<true>);
   set((const void*)k_ko_stage_bt_slab<false>);
+  auto raise = [&](const void* k, int bytes) {
+    const cudaError_t r =
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) e = r;
+  };
+  raise((const void*)k_deriv<false, 18, 17>, kDvMaxSmem);
+  raise((const void*)k_deriv<false, 34, 9>, kDvMaxSmem);
+  raise((const void*)k_point, kStageBytes);
+  // The other kernels of a step read their neighbours through L1, and follow
+  // kernels whose shared memory leaves little of it: without the preference
+  // the split stays as those left it (three evolutions of 512 blocks of 16^3
+  // on three streams: 23.4 ms a step against 19.5).
+  constexpr int F = kFixedNX, M = kMergedNX, U = kColUnroll;
+  for (const void* k :
+       {(const void*)k_ko_stage_ls<F + 1, true, true, F>, (const void*)k_ko_stage_ls<F + 1, true, false, F>,
+        (const void*)k_ko_stage_ls<U, false, true, F>, (const void*)k_ko_stage_ls<U, false, false, F>,
+        (const void*)k_ko_stage_ls<U, true, true, 0>, (const void*)k_ko_stage_ls<U, true, false, 0>,
+        (const void*)k_ko_stage_ls<U, false, true, 0>, (const void*)k_ko_stage_ls<U, false, false, 0>,
+        (const void*)k_ko_stage_bt<F + 1, true, true, F>, (const void*)k_ko_stage_bt<F + 1, true, false, F>,
+        (const void*)k_ko_stage_bt<U, false, true, F>, (const void*)k_ko_stage_bt<U, false, false, F>,
+        (const void*)k_ko_stage_bt<U, true, true, 0>, (const void*)k_ko_stage_bt<U, true, false, 0>,
+        (const void*)k_ko_stage_bt<U, false, true, 0>, (const void*)k_ko_stage_bt<U, false, false, 0>,
+        (const void*)k_ko_rhs<F + 1, true, F>, (const void*)k_ko_rhs<U, false, F>,
+        (const void*)k_ko_rhs<U, true, 0>, (const void*)k_ko_rhs<U, false, 0>,
+        (const void*)k_exchange_interior<NVAR, F>, (const void*)k_exchange_interior<NVAR, 0>,
+        (const void*)k_exchange_ghosts<NVAR, F>, (const void*)k_exchange_ghosts<NVAR, 0>,
+        (const void*)k_exchange_interior<Z4C_NWEYL, F>, (const void*)k_exchange_interior<Z4C_NWEYL, 0>,
+        (const void*)k_exchange_ghosts<Z4C_NWEYL, F>, (const void*)k_exchange_ghosts<Z4C_NWEYL, 0>,
+        (const void*)k_bc_axis<F, 0>, (const void*)k_bc_axis<F, 1>, (const void*)k_bc_axis<F, 2>,
+        (const void*)k_bc_axis<M, 0>, (const void*)k_bc_axis<M, 1>, (const void*)k_bc_axis<M, 2>,
+        (const void*)k_bc_axis<0, 0>, (const void*)k_bc_axis<0, 1>, (const void*)k_bc_axis<0, 2>,
+        (const void*)k_alg_constr_boundary<F>, (const void*)k_alg_constr_boundary<M>,
+        (const void*)k_alg_constr_boundary<0>, (const void*)k_alg_constr<F>, (const void*)k_alg_constr<0>,
+        (const void*)k_z4c_to_adm, (const void*)k_adm_to_z4c_gam, (const void*)k_adm_constraints<F>,
+        (const void*)k_adm_constraints<0>, (const void*)k_prep<F>, (const void*)k_prep<M>,
+        (const void*)k_prep<0>, (const void*)k_ricci<128, F>, (const void*)k_ricci<128, 0>}) {
+    const cudaError_t r = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                               cudaSharedmemCarveoutMaxL1);
+    if (e == cudaSuccess) e = r;
+  }
+  if (e == cudaSuccess) e = (cudaError_t)allow_deriv_smem_fast();
   return (int)e;
 }
 
-// MINB: CTAs per SM the heavy passes are compiled for (1: up to 255
-// registers per thread; kPointMinb(T): 168, three resident CTAs of 128 or
-// six of 64, for 1.5x the warps at a few dozen bytes of spill).
-template <int T, int MINB>
-static void launch_point_passes_t(const Grid& g, const DevParams& P, const double* u,
-                                  const RhsScratch& sc, double* rhs, int block0, int nblk,
-                                  int which, cudaStream_t st) {
-  const int64_t n = interior_count(g) * nblk;
-  COUNTED
-  if (which == 0)
-    (has_fixed_geometry(g) ? k_ricci<T, kFixedNX, MINB> : k_ricci<T, 0, MINB>)<<<div_up(n, T), T,
-                                                                                0, st>>>(
-        g, P, u, sc.sd, sc.rsum, block0, nblk);
-  else
-    (has_fixed_geometry(g) ? k_main<T, kFixedNX, MINB> : k_main<T, 0, MINB>)<<<div_up(n, T), T,
-                                                                              0, st>>>(
-        g, P, u, sc.sd, sc.rsum, sc.lv, rhs, block0, nblk);
-}
-static void launch_point_pass(const Grid& g, const DevParams& P, const double* u,
-                              const RhsScratch& sc, double* rhs, int block0, int nblk, int which,
-                              const LaunchShape& sh, cudaStream_t st) {
-  const bool hi = sh.point_regs == kPointRegsHigh && has_fixed_geometry(g);
-  switch (sh.point_threads) {
-    case 64:
-      if (hi) launch_point_passes_t<64, 6>(g, P, u, sc, rhs, block0, nblk, which, st);
-      else launch_point_passes_t<64, 1>(g, P, u, sc, rhs, block0, nblk, which, st);
-      break;
-    case 256: launch_point_passes_t<256, 1>(g, P, u, sc, rhs, block0, nblk, which, st); break;
-    default:
-      if (hi) launch_point_passes_t<128, 3>(g, P, u, sc, rhs, block0, nblk, which, st);
-      else launch_point_passes_t<128, 1>(g, P, u, sc, rhs, block0, nblk, which, st);
-      break;
-  }
-}
-
-// The right-hand side passes shared by every RHS launch: stored first
-// derivatives (sd), Ricci (rsum), advection sums (lv) and the main pass into
-// rhs (without KO).
+// The right-hand side without KO into rhs: the derivative pass, then the
+// pointwise pass, in pieces that fit the scratch.
 static void launch_rhs_passes(const Grid& g, const DevParams& P, const double* u,
                               const RhsScratch& sc, double* rhs, int block0, int nblk,
-                              const LaunchShape& sh, cudaStream_t st) {
-  size_t smem;
-  const SlabGeom S = slab_geom(g, sh, &smem);
-  const int ct = sh.column_threads;
-  if (S.kper > 0) {
-    // advection sums and stored first derivatives from shared-memory slabs
-    const dim3 grid((g.nx[2] + S.kper) / S.kper, NVAR, nblk);
+                              cudaStream_t st) {
+  for_deriv_chunks(g, nblk, sc, [&](int b, int nb, int ks, int nk) {
+    const DerivLaunch L = deriv_launch(g, nb, ks, nk);
     COUNTED
-    k_adv_prep_slab<<<grid, ct, smem, st>>>(g, P, u, sc.lv, sc.sd, S, block0);
-    launch_point_pass(g, P, u, sc, rhs, block0, nblk, 0, sh, st);
-  } else {
-    const int64_t cprep = (int64_t)(g.nx[0] + 7) * (g.nx[1] + 7);  // widest component region
+    (L.narrow ? k_deriv<false, 18, 17> : k_deriv<false, 34, 9>)<<<L.grid, L.threads, L.smem,
+                                                                  st>>>(g, P, u, sc.base, L.T,
+                                                                        block0 + b);
+    const int64_t np = (int64_t)nk * (g.nx[1] + 1) * (g.nx[0] + 1);
     COUNTED
-    (has_fixed_geometry(g) ? k_prep<kFixedNX>
-                         : has_merged_geometry(g) ? k_prep<kMergedNX> : k_prep<0>)<<<dim3(div_up(cprep, kPointThreads),
-                                                                 kSdComponents, nblk),
-                                                            kPointThreads, 0, st>>>(
-        g, P, u, sc.sd, block0);
-    launch_point_pass(g, P, u, sc, rhs, block0, nblk, 0, sh, st);
-    COUNTED
-    (has_fixed_geometry(g) ? k_adv<kFixedNX + 1, kFixedNX> : k_adv<kColUnroll, 0>)<<<div_up(columns(g, nblk), ct), ct,
-                                                                   0, st>>>(g, P, u, sc.lv, block0,
-                                                                            nblk);
-  }
-  launch_point_pass(g, P, u, sc, rhs, block0, nblk, 1, sh, st);
+    k_point<<<dim3(div_up(np, kDvGroup), nb), kDvGroup, kStageBytes, st>>>(
+        g, P, u, sc.base, rhs, block0 + b, ks, nk);
+  });
 }
 
 void launch_prep(const Grid& g, const DevParams& P, const double* u, double* sd, int block0,
@@ -1404,16 +1302,19 @@ void launch_prep(const Grid& g, const DevParams& P, const double* u, double* sd,
 void launch_prep_ricci(const Grid& g, const DevParams& P, const double* u, const RhsScratch& sc,
                        int block0, int nblk, const LaunchShape& sh, cudaStream_t st) {
   launch_prep(g, P, u, sc.sd, block0, nblk, st);
-  launch_point_pass(g, P, u, sc, nullptr, block0, nblk, 0, sh, st);
+  const dim3 grid(div_up(interior_count(g), 128), nblk);
+  COUNTED
+  (has_fixed_geometry(g) ? k_ricci<128, kFixedNX> : k_ricci<128, 0>)<<<grid, 128, 0, st>>>(
+      g, P, u, sc.sd, sc.rsum, block0);
 }
 
 void launch_rhs(const Grid& g, const DevParams& P, const double* u, const RhsScratch& sc,
                 double* rhs, int block0, int nblk, const LaunchShape& sh, cudaStream_t st) {
   if (sh.contract && !g.has_sommerfeld) {
-    launch_rhs_fast(g, P, u, sc, rhs, block0, nblk, sh, st);
+    launch_rhs_fast(g, P, u, sc, rhs, block0, nblk, st);
     return;
   }
-  launch_rhs_passes(g, P, u, sc, rhs, block0, nblk, sh, st);
+  launch_rhs_passes(g, P, u, sc, rhs, block0, nblk, st);
   size_t smem;
   const SlabGeom S = slab_geom(g, sh, &smem);
   const int ct = sh.column_threads;
@@ -1422,9 +1323,12 @@ void launch_rhs(const Grid& g, const DevParams& P, const double* u, const RhsScr
     k_ko_rhs_slab<<<dim3((g.nx[2] + S.kper) / S.kper, NVAR, nblk), ct, smem, st>>>(g, P, u, rhs,
                                                                                  S, block0);
   } else {
-    (has_fixed_geometry(g) ? k_ko_rhs<kFixedNX + 1, kFixedNX> : k_ko_rhs<kColUnroll, 0>)<<<div_up(columns(g, nblk), ct),
-                                                                        ct, 0, st>>>(g, P, u, rhs,
-                                                                                     block0, nblk);
+    const ColLaunch C = column_launch(g, nblk, ct);
+    constexpr int F = kFixedNX, U = kColUnroll;
+    const bool whole = C.T.n == 1;
+    (has_fixed_geometry(g) ? (whole ? k_ko_rhs<F + 1, true, F> : k_ko_rhs<U, false, F>)
+     : whole               ? k_ko_rhs<U, true, 0>
+                           : k_ko_rhs<U, false, 0>)<<<C.grid, ct, 0, st>>>(g, P, u, rhs, block0, nblk, C.T);
   }
 }
 
@@ -1432,10 +1336,10 @@ void launch_stage_ls(const Grid& g, const DevParams& P, const double* u, const R
                      double* rhs, double* u1, double* u_out, const LsStage& w, int block0,
                      int nblk, const LaunchShape& sh, cudaStream_t st) {
   if (sh.contract && !g.has_sommerfeld) {
-    launch_stage_ls_fast(g, P, u, sc, rhs, u1, u_out, w, block0, nblk, sh, st);
+    launch_stage_ls_fast(g, P, u, sc, rhs, u1, u_out, w, block0, nblk, st);
     return;
   }
-  launch_rhs_passes(g, P, u, sc, rhs, block0, nblk, sh, st);
+  launch_rhs_passes(g, P, u, sc, rhs, block0, nblk, st);
   size_t smem;
   const SlabGeom S = slab_geom(g, sh, &smem);
   const int ct = sh.column_threads;
@@ -1445,11 +1349,16 @@ void launch_stage_ls(const Grid& g, const DevParams& P, const double* u, const R
     kern<<<dim3((g.nx[2] + S.kper) / S.kper, NVAR, nblk), ct, smem, st>>>(g, P, u, rhs, u1, u_out,
                                                                         w, S, block0);
   } else {
-    auto kern = has_fixed_geometry(g)
-                    ? (g.has_sommerfeld ? k_ko_stage_ls<kFixedNX + 1, true, kFixedNX>
-                                        : k_ko_stage_ls<kFixedNX + 1, false, kFixedNX>)
-                    : (g.has_sommerfeld ? k_ko_stage_ls<kColUnroll, true, 0> : k_ko_stage_ls<kColUnroll, false, 0>);
-    kern<<<div_up(columns(g, nblk), ct), ct, 0, st>>>(g, P, u, rhs, u1, u_out, w, block0, nblk);
+    const ColLaunch C = column_launch(g, nblk, ct);
+    constexpr int F = kFixedNX, U = kColUnroll;
+    const bool som = g.has_sommerfeld, whole = C.T.n == 1;
+    auto kern =
+        has_fixed_geometry(g)
+            ? (whole ? (som ? k_ko_stage_ls<F + 1, true, true, F> : k_ko_stage_ls<F + 1, true, false, F>)
+                     : (som ? k_ko_stage_ls<U, false, true, F> : k_ko_stage_ls<U, false, false, F>))
+            : (whole ? (som ? k_ko_stage_ls<U, true, true, 0> : k_ko_stage_ls<U, true, false, 0>)
+                     : (som ? k_ko_stage_ls<U, false, true, 0> : k_ko_stage_ls<U, false, false, 0>));
+    kern<<<C.grid, ct, 0, st>>>(g, P, u, rhs, u1, u_out, w, block0, nblk, C.T);
   }
 }
 
@@ -1457,7 +1366,7 @@ void launch_stage_bt(const Grid& g, const DevParams& P, const double* u, const R
                      double* rhs, const double* un, double* const* k, double* u_out,
                      const BtStage& w, int block0, int nblk, const LaunchShape& sh,
                      cudaStream_t st) {
-  launch_rhs_passes(g, P, u, sc, rhs, block0, nblk, sh, st);
+  launch_rhs_passes(g, P, u, sc, rhs, block0, nblk, st);
   KPtrs K;
   for (int s = 0; s < 4; ++s) K.k[s] = k[s];
   size_t smem;
@@ -1469,14 +1378,20 @@ void launch_stage_bt(const Grid& g, const DevParams& P, const double* u, const R
     kern<<<dim3((g.nx[2] + S.kper) / S.kper, NVAR, nblk), ct, smem, st>>>(g, P, u, rhs, un, K,
                                                                         u_out, w, S, block0);
   } else {
-    auto kern = has_fixed_geometry(g)
-                    ? (g.has_sommerfeld ? k_ko_stage_bt<kFixedNX + 1, true, kFixedNX>
-                                        : k_ko_stage_bt<kFixedNX + 1, false, kFixedNX>)
-                    : (g.has_sommerfeld ? k_ko_stage_bt<kColUnroll, true, 0> : k_ko_stage_bt<kColUnroll, false, 0>);
-    kern<<<div_up(columns(g, nblk), ct), ct, 0, st>>>(g, P, u, rhs, un, K, u_out, w, block0,
-                                                      nblk);
+    const ColLaunch C = column_launch(g, nblk, ct);
+    constexpr int F = kFixedNX, U = kColUnroll;
+    const bool som = g.has_sommerfeld, whole = C.T.n == 1;
+    auto kern =
+        has_fixed_geometry(g)
+            ? (whole ? (som ? k_ko_stage_bt<F + 1, true, true, F> : k_ko_stage_bt<F + 1, true, false, F>)
+                     : (som ? k_ko_stage_bt<U, false, true, F> : k_ko_stage_bt<U, false, false, F>))
+            : (whole ? (som ? k_ko_stage_bt<U, true, true, 0> : k_ko_stage_bt<U, true, false, 0>)
+                     : (som ? k_ko_stage_bt<U, false, true, 0> : k_ko_stage_bt<U, false, false, 0>));
+    kern<<<C.grid, ct, 0, st>>>(g, P, u, rhs, un, K, u_out, w, block0, nblk, C.T);
   }
 }
+
+int64_t rhs_scratch_doubles(const Grid& g) { return dv_doubles(interior_count(g)); }
 
 // Slot of every direction in the neighbour list (mesh_topology.cpp:329-960
 // order, the c_dirs table of the context), indexed (o0+1) + 3(o1+1) + 9(o2+1).

@@ -52,31 +52,34 @@ long long kernel_launch_count();
 void add_kernel_launches(long long n);
 
 // All launches return cudaGetLastError() mapped by the caller.
-// Scratch of the right-hand-side passes, indexed by absolute block:
-// sd [block][33][vertex] (stored first derivatives of chi, g~, alpha, beta
-// along x, y, z), rsum [block][6][interior vertex] (R_ab + Rphi_ab),
-// lv [block][22][interior vertex] (advection sums).
+// Scratch of the right-hand-side passes: base, cap doubles, holds what the
+// derivative pass leaves for the pointwise pass (z4c_deriv.cuh), in pieces
+// where it does not hold the whole mesh.  The diagnostics and the adjoint use
+// the same memory, by absolute block, as sd [block][33][vertex] (stored first
+// derivatives of chi, g~, alpha, beta along x, y, z), rsum [block][6][interior
+// vertex] (R_ab + Rphi_ab) and lv [block][22][interior vertex].
 struct RhsScratch {
   double* sd;
   double* rsum;
   double* lv;
+  double* base;
+  int64_t cap;
 };
 constexpr int kSdComponents = 33;
+// Scratch doubles per block of the derivative pass.
+int64_t rhs_scratch_doubles(const Grid& g);
 
-// Launch shape of the right-hand-side passes: threads per CTA of the heavy
-// per-vertex passes (64, 128, 256), threads per CTA of the per-variable
-// passes (128, 256, 512) and the number of z-slabs per block in which those
-// passes stage a variable in shared memory (1-4; 0 or a slab whose planes do
-// not fit: global-memory pencils instead).
+// Launch shape of the right-hand-side passes: threads per CTA of the
+// Kreiss-Oliger and stage pass (128, 256, 512) and the number of z-slabs per
+// block in which it stages a variable in shared memory (1-4; 0 or a slab
+// whose planes do not fit: global-memory pencils instead).  point_threads and
+// point_regs are accepted and reported; the pointwise pass runs one warp per
+// CTA whatever they are.
 // contract: the contracted path (z4c_fast.cu) on meshes without
 // gr_sommerfeld faces: floating-point contraction, and the advection sums,
-// the Kreiss-Oliger terms and the stage update in one per-variable column
-// pass after the main pass; the right-hand side agrees with the exact path to
-// round-off instead of bit for bit.
-// point_regs: register budget of the heavy per-vertex passes on fixed-geometry
-// meshes: 0 (up to 255 per thread, two CTAs of 128 per SM) or
-// kPointRegsHigh (168: three CTAs of 128 or six of 64 per SM, 1.5x the
-// resident warps); point_threads 256 always takes 255.
+// the Kreiss-Oliger terms and the stage update in the derivative and pointwise
+// passes; the right-hand side agrees with the exact path to round-off instead
+// of bit for bit.
 constexpr int kPointRegsHigh = 168;
 struct LaunchShape {
   int point_threads = 128;
@@ -92,17 +95,17 @@ bool slabs_fit(const Grid& g, const LaunchShape& sh);
 // device before the first launch, outside stream capture); returns a
 // cudaError_t value.
 int allow_slab_smem();
+int allow_deriv_smem_fast();  // the contracted unit's part of it
 
-// Every RHS launch runs five kernels: stored first derivatives, Ricci pass,
-// advection sums, main pass (into rhs, without Kreiss-Oliger), then
-// Kreiss-Oliger fused with the consumer: in place for launch_rhs, with the
-// stage update for the stage launches (rhs then holds the pre-dissipation
-// right-hand side).
+// Every RHS launch runs the derivative pass, the pointwise pass (into rhs,
+// without Kreiss-Oliger), then Kreiss-Oliger fused with the consumer: in place
+// for launch_rhs, with the stage update for the stage launches (rhs then holds
+// the pre-dissipation right-hand side).
 void launch_rhs(const Grid& g, const DevParams& P, const double* u, const RhsScratch& sc,
                 double* rhs, int block0, int nblk, const LaunchShape& sh, cudaStream_t st);
-// The first two passes alone: the stored first derivatives of u into sc.sd
-// and the Ricci sums into sc.rsum (the linearisation point of the adjoint),
-// or the stored first derivatives alone into sd.
+// The adjoint's linearisation point: the stored first derivatives of u into
+// sc.sd and the Ricci sums into sc.rsum, or the stored first derivatives
+// alone into sd.
 void launch_prep_ricci(const Grid& g, const DevParams& P, const double* u, const RhsScratch& sc,
                        int block0, int nblk, const LaunchShape& sh, cudaStream_t st);
 void launch_prep(const Grid& g, const DevParams& P, const double* u, double* sd, int block0,
@@ -110,18 +113,16 @@ void launch_prep(const Grid& g, const DevParams& P, const double* u, double* sd,
 void launch_stage_ls(const Grid& g, const DevParams& P, const double* u, const RhsScratch& sc,
                      double* rhs, double* u1, double* u_out, const LsStage& w, int block0,
                      int nblk, const LaunchShape& sh, cudaStream_t st);
-// The contracted path (LaunchShape::contract): four launches, stored first
-// derivatives (exact), Ricci, the main pass into rhs without the advection
-// sums and Kreiss-Oliger, then one column pass that adds both and runs the
-// stage update (launch_stage_ls_fast) or writes the right-hand side back
+// The contracted path (LaunchShape::contract): the derivative pass, which
+// also forms the advection and Kreiss-Oliger sums, then the pointwise pass
+// with the stage update (launch_stage_ls_fast) or the right-hand side into rhs
 // (launch_rhs_fast).  Not for meshes with gr_sommerfeld faces (the launchers
 // above fall back to the exact path).
 void launch_stage_ls_fast(const Grid& g, const DevParams& P, const double* u,
                           const RhsScratch& sc, double* rhs, double* u1, double* u_out,
-                          const LsStage& w, int block0, int nblk, const LaunchShape& sh,
-                          cudaStream_t st);
+                          const LsStage& w, int block0, int nblk, cudaStream_t st);
 void launch_rhs_fast(const Grid& g, const DevParams& P, const double* u, const RhsScratch& sc,
-                     double* rhs, int block0, int nblk, const LaunchShape& sh, cudaStream_t st);
+                     double* rhs, int block0, int nblk, cudaStream_t st);
 void launch_stage_bt(const Grid& g, const DevParams& P, const double* u, const RhsScratch& sc,
                      double* rhs, const double* un, double* const* k, double* u_out,
                      const BtStage& w, int block0, int nblk, const LaunchShape& sh,

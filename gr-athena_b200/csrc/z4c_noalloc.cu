@@ -156,6 +156,8 @@ extern "C" int z4c_rhs_noalloc(const double* u, double* rhs, int nblocks, const 
   sc.sd = base + kFdBytes / sizeof(double);
   sc.rsum = sc.sd + (size_t)kSdComponents * g.nvol * chunk;
   sc.lv = sc.rsum + (size_t)6 * npts * chunk;
+  sc.base = sc.sd;
+  sc.cap = (int64_t)(room / sizeof(double));
 
   // FD scalings of finite_differencing.tpp:20-56, as z4c_create computes them
   FdScale f;

@@ -3,30 +3,24 @@
 // (z4c/adm_z4c.cpp:972-1037) evaluated in place from the state, constant-eta
 // branch, vacuum (matter terms vanish), Kreiss-Oliger dissipation included.
 //
-// The first derivatives that the reference stores in PrepareZ4cDerivatives
-// (chi, g~_ab, alpha, beta^a along every direction, on the interior extended
-// by 3 vertices across) are computed by a separate pass into the `sd`
-// scratch, exactly as the reference computes them; the passes below read
-// them there, both as first derivatives and as the inputs of the mixed
-// second derivatives (Dx_a of the stored Dx_b, Q1 of the reference).
-//
-// The work per vertex is split in two passes so that each keeps its live
-// values in registers:
+// The derivatives come from a source: the scratch that the derivative pass
+// leaves (DerivSrc; the mixed second derivatives are D_a of D_b, a < b, formed
+// as the reference forms them from its stored first derivatives), or, for the
+// adjoint's Ricci sums, the state and its stored first derivatives
+// (StencilSrc).
 //   ricci_point  the Ricci tensor of the conformal metric and its
-//                conformal-factor part, stored as Rsum_ab = R_ab + Rphi_ab
+//                conformal-factor part, as Rsum_ab = R_ab + Rphi_ab
 //                (the reference only ever uses the sum, :603, :745);
-//   rhs_point    everything else, reading Rsum_ab and the advection sums;
-// the advection sums (advect_point) and the Kreiss-Oliger terms (add_ko) run
-// in separate light kernels, one thread per vertex and variable.
+//   rhs_point    everything, without the Kreiss-Oliger terms.
 // The operation order of every quantity follows the reference line by line;
 // line numbers in the comments refer to calculate_z4c_rhs.cpp.
 #pragma once
 
 #include "z4c_common.cuh"
+#include "z4c_deriv.cuh"
 
 namespace z4c {
 
-#define UV(n) (U + (int64_t)(n) * nvol)
 #define GUU(a, b) g_uu[sidx(a, b)]
 
 // (a,b) of the symmetric pair q in xx,xy,xz,yy,yz,zz order
@@ -51,8 +45,108 @@ __device__ __forceinline__ double fd_d2(const double* __restrict__ f,
   if (a == b) return fd_dxx(f, s[a], F.cidx2[a]);
   return fd_dx(sdf + b * nvol, s[a], F.cidx1[a]);
 }
-#define SDF(slot) (SD + (int64_t)(slot) * 3 * nvol)
-#define SDV(slot, dir) __ldg(SD + ((int64_t)(slot) * 3 + (dir)) * nvol)
+// Load and store at a block-wide array's address, uniform over the CTA, plus
+// the thread's own 32-bit byte offset: the address of an operand is one
+// uniform addition and the thread keeps one offset register.
+__device__ __forceinline__ double ldo(const double* base, unsigned pb) {
+  return __ldg(reinterpret_cast<const double*>(reinterpret_cast<const char*>(base) + pb));
+}
+// The same for memory that the kernel also writes.
+__device__ __forceinline__ double ldm(const double* base, unsigned pb) {
+  return *reinterpret_cast<const double*>(reinterpret_cast<const char*>(base) + pb);
+}
+__device__ __forceinline__ void sto(double* base, unsigned pb, double v) {
+  *reinterpret_cast<double*>(reinterpret_cast<char*>(base) + pb) = v;
+}
+
+// Operands of the pointwise algebra at one interior vertex.  StencilSrc
+// evaluates the second derivatives of chi and g~ and the first ones of
+// Gamma~ from the state and its stored first derivatives (the linearisation
+// point of the adjoint); DerivSrc reads every derivative from the scratch of
+// the derivative pass (z4c_deriv.cuh).
+struct StencilSrc {
+  const double *U, *SD;
+  int64_t nvol;
+  const int64_t* s;
+  const FdScale* F;
+  unsigned pb;  // byte offset of the vertex in a variable
+  __device__ __forceinline__ double v(int n) const { return ldo(U + n * nvol, pb); }
+  __device__ __forceinline__ double d1(int slot, int dir) const {
+    return ldo(SD + (slot * 3 + dir) * nvol, pb);
+  }
+  __device__ __forceinline__ double dx(const double* f, int a) const {
+    double out = 0.;
+    out += -1. * (ldo(f - 3 * s[a], pb) - ldo(f + 3 * s[a], pb));
+    out += 9. * (ldo(f - 2 * s[a], pb) - ldo(f + 2 * s[a], pb));
+    out += -45. * (ldo(f - s[a], pb) - ldo(f + s[a], pb));
+    return out * F->cidx1[a];
+  }
+  __device__ __forceinline__ double d2(int slot, int q) const {
+    const int a = pair_a(q), b = pair_b(q);
+    if (a != b) return dx(SD + (slot * 3 + b) * nvol, a);
+    const double* f = U + sd_field_var(slot) * nvol;
+    double out = 0.;
+    out += 2. * (ldo(f - 3 * s[a], pb) + ldo(f + 3 * s[a], pb));
+    out += -27. * (ldo(f - 2 * s[a], pb) + ldo(f + 2 * s[a], pb));
+    out += 270. * (ldo(f - s[a], pb) + ldo(f + s[a], pb));
+    out += -490. * ldo(f, pb);
+    return out * F->cidx2[a];
+  }
+  __device__ __forceinline__ double dgam(int c, int b) const {
+    return dx(U + (Z4C_GAMX + c) * nvol, b);
+  }
+  __device__ __forceinline__ double dkhat(int b) const { return dx(U + Z4C_KHAT * nvol, b); }
+  __device__ __forceinline__ double dtheta(int b) const { return dx(U + Z4C_THETA * nvol, b); }
+};
+// A warp's 32 vertices: every derivative and the state's 22 variables staged
+// in shared memory, [component][vertex] and [variable][vertex].
+struct DerivSrc {
+  const double *U, *D;  // this lane's entry of the first row of each
+  __device__ __forceinline__ double v(int n) const { return U[n * kDvGroup]; }
+  __device__ __forceinline__ double c(int q) const { return D[q * kDvGroup]; }
+  __device__ __forceinline__ double d1(int slot, int dir) const { return c(9 * slot + dir); }
+  __device__ __forceinline__ double d2(int slot, int q) const { return c(9 * slot + 3 + q); }
+  __device__ __forceinline__ double dkhat(int b) const { return c(kDvKhat + b); }
+  __device__ __forceinline__ double dtheta(int b) const { return c(kDvTheta + b); }
+  __device__ __forceinline__ double dgam(int k, int b) const { return c(kDvGam + 3 * k + b); }
+  __device__ __forceinline__ double adv(int n) const { return c(kDvAdv + n); }
+};
+constexpr int kStageDoubles = (kDvComponents + NVAR) * kDvGroup;  // of one warp
+constexpr int kStageBytes = kStageDoubles * (int)sizeof(double);
+
+// Copies the first NC components of the warp's group (contiguous at D, 16-byte
+// aligned) into sm, asynchronously and all at once, so that the whole piece is
+// in flight however few warps the registers admit.
+template <int NC>
+__device__ __forceinline__ void stage_components(double* sm, const double* __restrict__ D) {
+  constexpr int pieces = NC * kDvGroup / 2;
+  const int lane = (int)threadIdx.x % kDvGroup;
+  const unsigned s = (unsigned)__cvta_generic_to_shared(sm);
+#pragma unroll 17
+  for (int q = lane; q < pieces; q += 32)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s + 16u * q), "l"(D + 2 * q)
+                 : "memory");
+}
+// All of them and this lane's 22 variables (at u + n nvol, if the lane holds a
+// vertex) behind them.
+__device__ __forceinline__ DerivSrc stage_group(double* sm, const double* __restrict__ D,
+                                                const double* __restrict__ u, int64_t nvol,
+                                                bool active) {
+  const int lane = (int)threadIdx.x % kDvGroup;
+  stage_components<kDvComponents>(sm, D);
+  double* su = sm + kDvComponents * kDvGroup + lane;
+  if (active) {
+    const unsigned t = (unsigned)__cvta_generic_to_shared(su);
+#pragma unroll
+    for (int n = 0; n < NVAR; ++n)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(t + 8u * kDvGroup * n),
+                   "l"(u + n * nvol)
+                   : "memory");
+  }
+  asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
+  __syncwarp();
+  return DerivSrc{su, sm + lane};
+}
 
 // The heavy derivative gathers below run as rolled loops (GATHER_LOOP)
 // writing small per-thread arrays; the tensor algebra that consumes them is
@@ -71,8 +165,8 @@ __device__ __forceinline__ double fd_d2(const double* __restrict__ f,
 
 // Inverse conformal metric (:295-311) and Christoffel symbols (:317-352).
 // Gamma_ddd is written only when the caller passes storage for it.
-__device__ __forceinline__ void christoffel(const double* __restrict__ SD, int64_t nvol,
-                                            const double g_dd[6], double g_uu[6],
+template <class Src>
+__device__ __forceinline__ void christoffel(const Src& src, const double g_dd[6], double g_uu[6],
                                             double Gamma_ddd[3][6], double Gamma_udd[3][6],
                                             double Gamma_u[3]) {
   {
@@ -85,7 +179,7 @@ __device__ __forceinline__ void christoffel(const double* __restrict__ SD, int64
 #pragma unroll
     for (int q = 0; q < 6; ++q)
 #pragma unroll
-      for (int c = 0; c < 3; ++c) dg[c][q] = SDV(kSdG + q, c);
+      for (int c = 0; c < 3; ++c) dg[c][q] = src.d1(kSdG + q, c);
 #pragma unroll
     for (int c = 0; c < 3; ++c)
 #pragma unroll
@@ -123,20 +217,17 @@ __device__ __forceinline__ void christoffel(const double* __restrict__ SD, int64
   }
 }
 
-// Rsum_ab = R_ab + Rphi_ab at one interior vertex (:357-458).
-__device__ __forceinline__ void ricci_point(const double* __restrict__ u,
-                                            const double* __restrict__ sd, int64_t nvol,
-                                            int64_t p, const int64_t s[3],
-                                            const DevParams& P, const FdScale& F,
+// Rsum_ab = R_ab + Rphi_ab at one interior vertex (:357-458), with the
+// metric's algebra (inverse, Gamma^c_ab, Gamma^c) it forms on the way.
+template <class Src>
+__device__ __forceinline__ void ricci_point(const Src& src, const z4c_params_t& opt,
+                                            double g_dd[6], double g_uu[6],
+                                            double Gamma_udd[3][6], double Gamma_u[3],
                                             double Rsum[6]) {
-  const z4c_params_t& opt = P.p;
-  const double* U = u + p;
-  const double* SD = sd + p;
-  double g_dd[6];
 #pragma unroll
-  for (int c = 0; c < 6; ++c) g_dd[c] = __ldg(UV(Z4C_GXX + c));
-  double g_uu[6], Gamma_ddd[3][6], Gamma_udd[3][6], Gamma_u[3];
-  christoffel(SD, nvol, g_dd, g_uu, Gamma_ddd, Gamma_udd, Gamma_u);
+  for (int c = 0; c < 6; ++c) g_dd[c] = src.v(Z4C_GXX + c);
+  double Gamma_ddd[3][6];
+  christoffel(src, g_dd, g_uu, Gamma_ddd, Gamma_udd, Gamma_u);
 #define GDDD(c, a, b) Gamma_ddd[c][sidx(a, b)]
 #define GUDD(c, a, b) Gamma_udd[c][sidx(a, b)]
 
@@ -145,9 +236,8 @@ __device__ __forceinline__ void ricci_point(const double* __restrict__ u,
   double dGam[3][3];  // [b][c] = d_b Gamma^c
 GATHER_LOOP
   for (int c = 0; c < 3; ++c) {
-    const double* f = UV(Z4C_GAMX + c);
 #pragma unroll
-    for (int b = 0; b < 3; ++b) dGam[b][c] = fd_dx(f, s[b], F.cidx1[b]);
+    for (int b = 0; b < 3; ++b) dGam[b][c] = src.dgam(c, b);
   }
   double R_dd[6];
 #pragma unroll
@@ -164,14 +254,12 @@ GATHER_LOOP
   // ddg_dddd(c,d,a,b): second derivative along c,d of g_ab, :158-178
 GATHER_LOOP
   for (int q = 0; q < 6; ++q) {
-    const double* f = UV(Z4C_GXX + q);
-    const double* sdf = SDF(kSdG + q);
     double sacc = R_dd[q];
 #pragma unroll
     for (int c = 0; c < 3; ++c)
 #pragma unroll
       for (int d = c; d < 3; ++d)
-        sacc -= ((c == d) ? 0.5 : 1.0) * GUU(c, d) * fd_d2(f, sdf, nvol, sidx(c, d), s, F);
+        sacc -= ((c == d) ? 0.5 : 1.0) * GUU(c, d) * src.d2(kSdG + q, sidx(c, d));
     R_dd[q] = sacc;
   }
 #pragma unroll
@@ -191,16 +279,16 @@ GATHER_LOOP
     }
 
   // conformal-factor part, :241-245, :402-458
-  const double chi = __ldg(UV(Z4C_CHI));
+  const double chi = src.v(Z4C_CHI);
   const double chi_guarded = dmax(chi, opt.chi_div_floor);
   const double oochi = 1.0 / chi_guarded;
   const double oochi_psi_power = 1.0 / opt.chi_psi_power;
   double dphi_d[3];
 #pragma unroll
-  for (int a = 0; a < 3; ++a) dphi_d[a] = SDV(kSdChi, a) * oochi * oochi_psi_power;
+  for (int a = 0; a < 3; ++a) dphi_d[a] = src.d1(kSdChi, a) * oochi * oochi_psi_power;
   double ddchi[6];  // stored ddchi_dd_3d
 GATHER_LOOP
-  for (int q = 0; q < 6; ++q) ddchi[q] = fd_d2(UV(Z4C_CHI), SDF(kSdChi), nvol, q, s, F);
+  for (int q = 0; q < 6; ++q) ddchi[q] = src.d2(kSdChi, q);
   double Ddphi_dd[6];
 #pragma unroll
   for (int a = 0; a < 3; ++a)
@@ -232,32 +320,18 @@ GATHER_LOOP
 }
 
 // The 22 right-hand-side values at one interior vertex without the
-// Kreiss-Oliger terms, given Rsum_ab (rsum[q * stride]) and the advection sums
-// (lv[n * stride]).  With LV = false the advection sums are left out (read
-// as zero; lv is not read): the contracted path adds them, scaled, with the
-// Kreiss-Oliger terms afterwards.
-template <bool LV = true>
-__device__ __forceinline__ void rhs_point(const double* __restrict__ u,
-                                          const double* __restrict__ sd, int64_t nvol,
-                                          int64_t p, const int64_t s[3],
-                                          const DevParams& P, const FdScale& F,
-                                          const double* __restrict__ rsum,
-                                          const double* __restrict__ lv, int64_t stride,
+// Kreiss-Oliger terms.  With LV = false the advection sums are left out: the
+// contracted path adds them, scaled, with the Kreiss-Oliger terms afterwards.
+template <bool LV, class Src>
+__device__ __forceinline__ void rhs_point(const Src& src, const z4c_params_t& opt,
                                           double out[NVAR]) {
-  const z4c_params_t& opt = P.p;
-  const double* U = u + p;
-  const double* SD = sd + p;
-  double g_dd[6], A_dd[6];
+  double g_dd[6], g_uu[6], Gamma_udd[3][6], Gamma_u[3], Rsum[6];
+  ricci_point(src, opt, g_dd, g_uu, Gamma_udd, Gamma_u, Rsum);
+  double A_dd[6];
 #pragma unroll
-  for (int c = 0; c < 6; ++c) {
-    g_dd[c] = __ldg(UV(Z4C_GXX + c));
-    A_dd[c] = __ldg(UV(Z4C_AXX + c));
-  }
-  const double chi = __ldg(UV(Z4C_CHI)), Khat = __ldg(UV(Z4C_KHAT));
-  const double Theta = __ldg(UV(Z4C_THETA)), alpha = __ldg(UV(Z4C_ALPHA));
-
-  double g_uu[6], Gamma_udd[3][6], Gamma_u[3];
-  christoffel(SD, nvol, g_dd, g_uu, nullptr, Gamma_udd, Gamma_u);
+  for (int c = 0; c < 6; ++c) A_dd[c] = src.v(Z4C_AXX + c);
+  const double chi = src.v(Z4C_CHI), Khat = src.v(Z4C_KHAT);
+  const double Theta = src.v(Z4C_THETA), alpha = src.v(Z4C_ALPHA);
 #define GUDD(c, a, b) Gamma_udd[c][sidx(a, b)]
 
   // :231-274
@@ -271,9 +345,9 @@ __device__ __forceinline__ void rhs_point(const double* __restrict__ u,
   double dchi_d[3], dphi_d[3], dalpha_d[3];
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    dchi_d[a] = SDV(kSdChi, a);
+    dchi_d[a] = src.d1(kSdChi, a);
     dphi_d[a] = dchi_d[a] * oochi * oochi_psi_power;
-    dalpha_d[a] = SDV(kSdAlpha, a);
+    dalpha_d[a] = src.d1(kSdAlpha, a);
   }
 
   // D D alpha, :482-521
@@ -284,7 +358,7 @@ __device__ __forceinline__ void rhs_point(const double* __restrict__ u,
     for (int d = 0; d < 3; ++d) Ddalpha += GUU(c, d) * dphi_d[c] * dalpha_d[d];
   double ddalpha[6];
 GATHER_LOOP
-  for (int q = 0; q < 6; ++q) ddalpha[q] = fd_d2(UV(Z4C_ALPHA), SDF(kSdAlpha), nvol, q, s, F);
+  for (int q = 0; q < 6; ++q) ddalpha[q] = src.d2(kSdAlpha, q);
   double Ddalpha_dd[6];
 #pragma unroll
   for (int a = 0; a < 3; ++a)
@@ -347,8 +421,8 @@ GATHER_LOOP
     double sacc = 0;
 #pragma unroll
     for (int b = 0; b < 3; ++b) {
-      const double dKhat_b = fd_dx(UV(Z4C_KHAT), s[b], F.cidx1[b]);
-      const double dTheta_b = fd_dx(UV(Z4C_THETA), s[b], F.cidx1[b]);
+      const double dKhat_b = src.dkhat(b);
+      const double dTheta_b = src.dtheta(b);
       sacc -= chi_pow_DA_u * A_uu[sidx(a, b)] * dchi_d[b] * oochi;
       sacc -= (1. / 3.) * GUU(a, b) * (2. * dKhat_b + dTheta_b);
     }
@@ -367,16 +441,16 @@ GATHER_LOOP
   for (int a = 0; a < 3; ++a)
 #pragma unroll
     for (int b = a; b < 3; ++b)
-      R += ((a == b) ? 1.0 : 2.0) * oopsi4 * GUU(a, b) * __ldg(rsum + sidx(a, b) * stride);
+      R += ((a == b) ? 1.0 : 2.0) * oopsi4 * GUU(a, b) * Rsum[sidx(a, b)];
   const double Ht = R + (2. / 3.) * (K * K) - trAA;
 
   // advective derivatives, :184-226
   double beta_u[3];
 #pragma unroll
-  for (int a = 0; a < 3; ++a) beta_u[a] = __ldg(UV(Z4C_BETAX + a));
+  for (int a = 0; a < 3; ++a) beta_u[a] = src.v(Z4C_BETAX + a);
   // the advection sums, each read where it enters (lv[n * stride])
   auto Lv = [&](int n) {
-    if constexpr (LV) return __ldg(lv + (int64_t)n * stride);
+    if constexpr (LV) return src.adv(n);
     else return 0.0;
   };
   double LGam_u[3], Lg_dd[6], LA_dd[6];
@@ -386,7 +460,7 @@ GATHER_LOOP
 #pragma unroll
   for (int a = 0; a < 3; ++a)
 #pragma unroll
-    for (int b = 0; b < 3; ++b) dbeta_du[b][a] = SDV(kSdBeta + a, b);
+    for (int b = 0; b < 3; ++b) dbeta_du[b][a] = src.d1(kSdBeta + a, b);
   double dbeta = 0;
 #pragma unroll
   for (int a = 0; a < 3; ++a) dbeta += dbeta_du[a][a];
@@ -395,7 +469,7 @@ GATHER_LOOP
 GATHER_LOOP
   for (int i = 0; i < 18; ++i) {
     const int c = i / 6, q = i % 6;
-    ddbeta[c][q] = fd_d2(UV(Z4C_BETAX + c), SDF(kSdBeta + c), nvol, q, s, F);
+    ddbeta[c][q] = src.d2(kSdBeta + c, q);
   }
   double ddbeta_d[3] = {0, 0, 0};
 #pragma unroll
@@ -441,7 +515,7 @@ GATHER_LOOP
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     double v = 2. * alpha * DA_u[a] + LGam_u[a];
-    v -= 2. * alpha * opt.damp_kappa1 * (__ldg(UV(Z4C_GAMX + a)) - Gamma_u[a]);
+    v -= 2. * alpha * opt.damp_kappa1 * (src.v(Z4C_GAMX + a) - Gamma_u[a]);
 #pragma unroll
     for (int b = 0; b < 3; ++b) v -= 2. * A_uu[sidx(a, b)] * dalpha_d[b];
     out[Z4C_GAMX + a] = v;
@@ -452,7 +526,7 @@ GATHER_LOOP
     for (int b = a; b < 3; ++b) {
       const int q = sidx(a, b);
       out[Z4C_GXX + q] = -2. * alpha * A_dd[q] + Lg_dd[q];
-      double v = oopsi4 * (-Ddalpha_dd[q] + alpha * __ldg(rsum + q * stride));
+      double v = oopsi4 * (-Ddalpha_dd[q] + alpha * Rsum[q]);
       v -= (1. / 3.) * g_dd[q] * (-Ddalpha + alpha * R);
       v += alpha * (K * A_dd[q] - 2. * AA_dd[q]);
       v += LA_dd[q];
@@ -464,7 +538,7 @@ GATHER_LOOP
   }
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    const double gam_a = __ldg(UV(Z4C_GAMX + a));
+    const double gam_a = src.v(Z4C_GAMX + a);
     double v = opt.shift_Gamma * gam_a + opt.shift_advect * Lv(Z4C_BETAX + a);
     if (fabs(opt.shift_alpha2Gamma) > 0.0) v += opt.shift_alpha2Gamma * (alpha * alpha) * gam_a;
     if (fabs(opt.shift_H) > 0.0) {
@@ -477,9 +551,6 @@ GATHER_LOOP
   }
 }
 
-#undef UV
-#undef SDF
-#undef SDV
 #undef GUU
 #undef GDD
 #undef ADD

@@ -9,24 +9,57 @@
 
 namespace z4c {
 
-// ---- per-variable passes: advection sums and Kreiss-Oliger -------------------
-// One thread per (block, variable, interior (i, j)) column, looping over the
-// interior k.  Stencils along x and y read their lines directly; along z the
-// nine-vertex window slides in registers.  Index arithmetic is 32-bit (the
-// launcher checks that the thread count fits).
-struct Column {
-  int b, n, i, j;
+// ---- per-variable pass: Kreiss-Oliger -------------------
+// One thread per (block, variable, interior (i, j)) column and chunk of
+// interior planes, looping over the chunk's k.  Stencils along x and y read
+// their lines directly; along z the nine-vertex window slides in registers.
+// Index arithmetic is 32-bit (the launcher checks that the thread count fits).
+struct ColChunks {
+  int kc;  // interior planes per thread
+  int n;   // chunks per column; 1: whole columns
 };
-__device__ __forceinline__ bool column_index(const Grid& g, int block0, int nblk, Column& c) {
+struct Column {
+  int b, n, i, j, k0, k1;
+};
+template <bool WHOLE>
+__device__ __forceinline__ bool column_index(const Grid& g, const ColChunks& T, int block0,
+                                             int nblk, Column& c) {
   const int n0 = g.nx[0] + 1, per = n0 * (g.nx[1] + 1);
   const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (t >= per * NVAR * nblk) return false;
-  const int ij = t % per, rest = t / per;
+  const int nc = WHOLE ? 1 : T.n;
+  if (t >= per * NVAR * nblk * nc) return false;
+  const int ij = t % per;
+  int rest = t / per;
+  c.k0 = NG;
+  c.k1 = NG + g.nx[2];
+  if constexpr (!WHOLE) {
+    c.k0 = NG + (rest % nc) * T.kc;
+    c.k1 = min(c.k0 + T.kc - 1, c.k1);
+    rest /= nc;
+  }
   c.n = rest % NVAR;
   c.b = block0 + rest / NVAR;
   c.i = NG + ij % n0;
   c.j = NG + ij / n0;
   return true;
+}
+// Columns are cut into chunks where there are too few of them to give every
+// SM 48 warps: the z loop of a column is a serial chain of loads (a 48^3 block,
+// low-storage stage: 331 us whole, 234 us in chunks; 16^3: 64 and 37).
+struct ColLaunch {
+  ColChunks T;
+  int grid;
+};
+inline ColLaunch column_launch(const Grid& g, int nblk, int threads) {
+  const int nk = g.nx[2] + 1;
+  const long long cols = (long long)(g.nx[0] + 1) * (g.nx[1] + 1) * NVAR * nblk;
+  long long chunks = (148LL * 48 * 32 + cols - 1) / cols;
+  if (chunks > nk) chunks = nk;
+  ColLaunch L;
+  L.T.kc = (int)((nk + chunks - 1) / chunks);
+  L.T.n = (nk + L.T.kc - 1) / L.T.kc;
+  L.grid = (int)((cols * L.T.n + threads - 1) / threads);
+  return L;
 }
 
 // Loads for the stencil helpers below: read-only cache path for global
@@ -37,55 +70,30 @@ __device__ __forceinline__ double ld(const double* p) {
   return *p;
 }
 
-// Lop-sided advection along one direction (FDStencilBiased{Left,Right}<1,4,2>,
-// finite_differencing.tpp:175-191): only the side the sign of vx selects is
-// evaluated; its value is the reference's, which evaluates both and keeps one.
-template <bool GL = true>
-__device__ __forceinline__ double fd_lx_side(const double* __restrict__ u, int st, double vx,
-                                             double lidx) {
-  if (vx < 0) {
-    double dl = 0.;
-    dl += 1. * ld<GL>(u - 4 * st);
-    dl += -8. * ld<GL>(u - 3 * st);
-    dl += 30. * ld<GL>(u - 2 * st);
-    dl += -80. * ld<GL>(u - st);
-    dl += 35. * ld<GL>(u);
-    dl += 24. * ld<GL>(u + st);
-    dl += -2. * ld<GL>(u + 2 * st);
-    return (vx * dl) * lidx;
-  }
-  double dr = 0.;
-  dr += -1. * ld<GL>(u + 4 * st);
-  dr += 8. * ld<GL>(u + 3 * st);
-  dr += -30. * ld<GL>(u + 2 * st);
-  dr += 80. * ld<GL>(u + st);
-  dr += -35. * ld<GL>(u);
-  dr += -24. * ld<GL>(u - st);
-  dr += 2. * ld<GL>(u - 2 * st);
-  return (vx * dr) * lidx;
+// w[0..8] = f(-4..4) along stride st, the centre c given.
+__device__ __forceinline__ void load_line(const double* __restrict__ f, int st, double c,
+                                          double w[9]) {
+#pragma unroll
+  for (int q = 0; q < 9; ++q) w[q] = q == 4 ? c : __ldg(f + (q - 4) * st);
 }
-// The same along z from the window w[0..8] = f(k-4..k+4).
-__device__ __forceinline__ double fd_lx_window(const double w[9], double vx, double lidx) {
-  if (vx < 0) {
-    double dl = 0.;
-    dl += 1. * w[0];
-    dl += -8. * w[1];
-    dl += 30. * w[2];
-    dl += -80. * w[3];
-    dl += 35. * w[4];
-    dl += 24. * w[5];
-    dl += -2. * w[6];
-    return (vx * dl) * lidx;
-  }
-  double dr = 0.;
-  dr += -1. * w[8];
-  dr += 8. * w[7];
-  dr += -30. * w[6];
-  dr += 80. * w[5];
-  dr += -35. * w[4];
-  dr += -24. * w[3];
-  dr += 2. * w[2];
-  return (vx * dr) * lidx;
+// Advection factor of variable n in the right-hand side (:860-902).
+__device__ __forceinline__ double adv_factor(const z4c_params_t& p, int n) {
+  if (n == Z4C_ALPHA) return p.lapse_advect;
+  if (n >= Z4C_BETAX && n <= Z4C_BETAZ) return p.shift_advect;
+  return 1.0;
+}
+
+// Advection and Kreiss-Oliger along one line w[0..8] = f(-4..4).  Half the
+// difference of the two lop-sided stencils is the Kreiss-Oliger stencil K and
+// half their sum the centred C below, so the side the sign of v selects is
+// (v C - |v| K) / 2: one pass over the taps gives both terms, without a
+// branch.  al = advection factor / (2 * 60 dx), kd the dissipation's factor.
+__device__ __forceinline__ double adv_ko_line(const double w[9], double v, double al, double kd) {
+  const double K = (w[0] + w[8]) - 8. * (w[1] + w[7]) + 28. * (w[2] + w[6]) -
+                   56. * (w[3] + w[5]) + 70. * w[4];
+  const double C = (w[0] - w[8]) - 8. * (w[1] - w[7]) + 32. * (w[2] - w[6]) -
+                   104. * (w[3] - w[5]);
+  return al * v * C + (kd - al * fabs(v)) * K;
 }
 
 // Kreiss-Oliger along one direction (FDStencilCenteredDegreeEven<8,4>,

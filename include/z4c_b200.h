@@ -372,33 +372,28 @@ int z4c_fp64_probe(z4c_ctx *ctx, double *tflops);
  * stage) instead of the batched launch inside z4c_stage/z4c_evolve. */
 int z4c_set_per_block(z4c_ctx *ctx, int per_block);
 /* Launch shape of the right-hand-side passes (no reference counterpart):
- * tile = {threads per CTA of the per-vertex Ricci and main passes (64, 128,
- * 256), threads per CTA of the per-variable passes (advection, stored first
- * derivatives, Kreiss-Oliger + stage update: 128, 256, 512), z-slabs per
- * MeshBlock in which those passes stage one variable in shared memory (1-4;
- * 0, or slabs whose vertex planes do not fit, selects global-memory
- * pencils)}.  The default is {128, 128, 0}; unsupported shapes return
- * Z4C_EINVAL.  Results do not depend on the shape. */
+ * tile = {64, 128 or 256 (kept for callers; the pointwise pass runs one warp
+ * per CTA), threads per CTA of the Kreiss-Oliger and stage pass (128, 256,
+ * 512), z-slabs per MeshBlock in which that pass stages one variable in shared
+ * memory (1-4; 0, or slabs whose vertex planes do not fit, selects
+ * global-memory pencils)}.  The default is {128, 128, 0}; unsupported shapes
+ * return Z4C_EINVAL.  Results do not depend on the shape. */
 int z4c_set_tile(z4c_ctx *ctx, int ti, int tj, int tk);
 int z4c_get_tile(const z4c_ctx *ctx, int tile_out[3]);
 /* Contracted right-hand side (no reference counterpart): with on != 0 every
  * later z4c_rhs, stage and step of the context takes the contracted path:
  * floating-point contraction (fused multiply-adds), the advection sums and
- * the Kreiss-Oliger terms added in one per-variable pass, and the stage
- * update fused with the main right-hand-side pass, four launches per stage.
+ * the Kreiss-Oliger terms formed with the derivatives, and the stage update
+ * fused with the pointwise right-hand-side pass, two launches per stage.
  * Its right-hand side agrees with the exact path's (which matches the
  * reference bit for bit) to round-off, within the 1e-12 relative bound per
  * evaluation; meshes with gr_sommerfeld faces and the Butcher integrator keep
  * the exact path.  Off by default; switching drops the captured step graph,
  * and the autotuner times the path that is switched on. */
 int z4c_set_contract(z4c_ctx *ctx, int on);
-/* Register budget of the heavy per-vertex right-hand-side passes on meshes of
- * 16^3 MeshBlocks (no reference counterpart): 0 lets them use up to 255
- * registers per thread (two CTAs of 128 threads per SM), 168 compiles them
- * for three CTAs of 128 or six of 64 per SM (1.5x the resident warps for a
- * few dozen bytes of spill); 256-thread CTAs always take 255.  The arithmetic
- * is the same either way.  The autotuner tries both; switching drops the
- * captured step graph. */
+/* Register budget of the per-vertex right-hand-side pass (no reference
+ * counterpart), 0 or 168: kept for callers and reported back; the pass has one
+ * instance, bound by memory, and results do not depend on it. */
 int z4c_set_point_regs(z4c_ctx *ctx, int regs);
 int z4c_get_point_regs(const z4c_ctx *ctx, int *regs);
 int z4c_get_contract(const z4c_ctx *ctx, int *on);
