@@ -82,8 +82,12 @@ __device__ __forceinline__ void adm_to_z4c_point(const z4c_params_t& opt, const 
 #undef A_
 }
 
-// ADMConstraints at one interior vertex; writes the 7 constraint values.
-__device__ __forceinline__ void adm_constraints_point(const double* __restrict__ uB,
+// ADMConstraints at one interior vertex; writes the 7 constraint values.  src
+// has the first and second derivatives of chi and g~ (d1, d2 of z4c_rhs.cuh's
+// DerivSrc).
+template <class Src>
+__device__ __forceinline__ void adm_constraints_point(const Src& src,
+                                                      const double* __restrict__ uB,
                                                       const double* __restrict__ admB,
                                                       int64_t nvol, int64_t p,
                                                       const int64_t s[3], const DevParams& P,
@@ -108,13 +112,13 @@ __device__ __forceinline__ void adm_constraints_point(const double* __restrict__
     gph[c] = __ldg(AV(Z4C_ADM_GXX + c));
   }
 #pragma unroll
-  for (int a = 0; a < 3; ++a) dchi[a] = fd_dx(UV(Z4C_CHI), s[a], F.cidx1[a]);
+  for (int a = 0; a < 3; ++a) dchi[a] = src.d1(0, a);
   // conformal first derivatives d_c g~_ab (stored dg_ddd_3d)
   double dg3[3][6];
 #pragma unroll
   for (int c = 0; c < 3; ++c)
 #pragma unroll
-    for (int q = 0; q < 6; ++q) dg3[c][q] = fd_dx(UV(Z4C_GXX + q), s[c], F.cidx1[c]);
+    for (int q = 0; q < 6; ++q) dg3[c][q] = src.d1(1 + q, c);
   // pass 1: physical first derivatives, :446-460 / :532-546
   double dg[3][6];
 #pragma unroll
@@ -154,14 +158,11 @@ __device__ __forceinline__ void adm_constraints_point(const double* __restrict__
   auto ddg = [&](int a, int b, int c, int d) -> double {
     const int ab_lo = a < b ? a : b, ab_hi = a < b ? b : a;
     const int q = sidx(c, d);
-    const double* f = UV(Z4C_GXX + q);
     const double dchi_a = dchi[ab_lo], dchi_b = dchi[ab_hi];
     const double gtil = gt[q];
-    double ddchi;
-    if (ab_lo == ab_hi) ddchi = fd_dxx(UV(Z4C_CHI), s[ab_lo], F.cidx2[ab_lo]);
-    else ddchi = fd_dxy(UV(Z4C_CHI), s[ab_lo], s[ab_hi], F.cidx1[ab_lo], F.cidx1[ab_hi]);
+    const double ddchi = src.d2(0, sidx(ab_lo, ab_hi));
+    const double ddg_conf = src.d2(1 + q, sidx(ab_lo, ab_hi));
     if (ab_lo == ab_hi) {
-      const double ddg_conf = fd_dxx(f, s[ab_lo], F.cidx2[ab_lo]);
       const double d3 = dg3[ab_lo][q];
       if (pw == -4.)
         return oochi * (ddg_conf - oochi * (2.0 * dchi_a * d3 + ddchi * gtil) +
@@ -170,7 +171,6 @@ __device__ __forceinline__ void adm_constraints_point(const double* __restrict__
       return psi4c * (ddg_conf + fac * oochi * (2.0 * dchi_a * d3 + ddchi * gtil) +
                       fac * fac2 * oochi * oochi * dchi_a * dchi_a * gtil);
     }
-    const double ddg_conf = fd_dxy(f, s[ab_lo], s[ab_hi], F.cidx1[ab_lo], F.cidx1[ab_hi]);
     const double dgb = dg3[ab_hi][q], dga = dg3[ab_lo][q];
     if (pw == -4.)
       return oochi * (ddg_conf - oochi * (dchi_a * dgb + dchi_b * dga + ddchi * gtil) +

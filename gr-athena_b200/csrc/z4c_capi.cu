@@ -859,9 +859,9 @@ int z4c_adm_constraints(z4c_ctx* ctx, int reg_con, int reg_adm, int reg_u, int b
       reg_nvar_(reg_u) != Z4C_NVAR)
     return fail(Z4C_EINVAL, "ADMConstraints needs con, adm and a Z4c register");
   if ((rc = check_block(ctx, block, &b0, &nb))) return rc;
-  launch_adm_constraints(ctx->g, ctx->dev(), ctx->reg[reg_adm], ctx->reg[reg_u],
-                         ctx->reg[reg_con], ctx->xf, b0, nb, ctx->stream);
-  LAUNCH_CHECK("adm_constraints");
+  CUDA_TRY((cudaError_t)launch_adm_constraints(ctx->g, ctx->dev(), ctx->scratch(),
+                                               ctx->reg[reg_adm], ctx->reg[reg_u],
+                                               ctx->reg[reg_con], ctx->xf, b0, nb, ctx->stream));
   return Z4C_OK;
 }
 
@@ -1402,9 +1402,9 @@ int merged_evolve(z4c_ctx* c, double dt, int nsteps, int with_constraints) {
   launch_z4c_to_adm(c->g, P, c->reg[Z4C_REG_U], c->reg[Z4C_REG_ADM], 0, c->g.nblocks, c->stream);
   LAUNCH_CHECK("z4c_to_adm");
   if (with_constraints) {
-    launch_adm_constraints(c->g, P, c->reg[Z4C_REG_ADM], c->reg[Z4C_REG_U],
-                           c->reg[Z4C_REG_CON], c->xf, 0, c->g.nblocks, c->stream);
-    LAUNCH_CHECK("constraints");
+    CUDA_TRY((cudaError_t)launch_adm_constraints(
+        c->g, P, c->scratch(), c->reg[Z4C_REG_ADM], c->reg[Z4C_REG_U], c->reg[Z4C_REG_CON], c->xf,
+        0, c->g.nblocks, c->stream));
   }
   if (c->ntrk > 0)
     CUDA_TRY(cudaMemcpyAsync(c->trk, m->trk, sizeof(double) * 8 * c->ntrk,
@@ -1459,9 +1459,9 @@ int z4c_evolve(z4c_ctx* ctx, double dt, int nsteps, int with_constraints) {
     if (nsteps == 0)
       launch_z4c_to_adm(ctx->g, P, ctx->reg[Z4C_REG_U], ctx->reg[Z4C_REG_ADM], 0, ctx->g.nblocks,
                         ctx->stream);
-    launch_adm_constraints(ctx->g, P, ctx->reg[Z4C_REG_ADM], ctx->reg[Z4C_REG_U],
-                           ctx->reg[Z4C_REG_CON], ctx->xf, 0, ctx->g.nblocks, ctx->stream);
-    LAUNCH_CHECK("constraints");
+    CUDA_TRY((cudaError_t)launch_adm_constraints(
+        ctx->g, P, ctx->scratch(), ctx->reg[Z4C_REG_ADM], ctx->reg[Z4C_REG_U],
+        ctx->reg[Z4C_REG_CON], ctx->xf, 0, ctx->g.nblocks, ctx->stream));
   }
   return Z4C_OK;
 }

@@ -157,9 +157,10 @@ void launch_z4c_to_adm(const Grid& g, const DevParams& P, const double* u, doubl
 // alg = 0 leaves out the final AlgConstr (the adjoint's recomputation)
 void launch_adm_to_z4c(const Grid& g, const DevParams& P, const double* adm, double* u,
                        double* guu_scratch, int block0, int nblk, cudaStream_t st, int alg = 1);
-void launch_adm_constraints(const Grid& g, const DevParams& P, const double* adm,
-                            const double* u, double* con, const double* xf, int block0,
-                            int nblk, cudaStream_t st);
+// Uses the right-hand-side scratch; returns a cudaError_t value.
+int launch_adm_constraints(const Grid& g, const DevParams& P, const RhsScratch& sc,
+                           const double* adm, const double* u, double* con, const double* xf,
+                           int block0, int nblk, cudaStream_t st);
 // Z4cWeyl on blocks [block0, block0+nblk): the stored first derivatives of u
 // into sd (k_prep), the curvature terms into the scratch rs (6 values per
 // interior vertex) and ks (22), then psi4 (2 variables) into weyl.
