@@ -479,57 +479,66 @@ __device__ int trk_lagrange1d(double origin, double delta, int siz, double coord
   return point;
 }
 
-// PunctureTracker::InterpolateShift (:95-129): one thread per tracker finds
-// the block that holds the puncture exclusively (MeshBlock::
-// PointContainedExclusive, mesh/meshblock.cpp:1186-1201) and interpolates
-// the shift there (LagrangeInterpND: x innermost, then y, then z).
-__global__ void k_track_interp(Grid g, DevParams P, const double* __restrict__ u,
-                               double* __restrict__ trk, int ntrk) {
+// PunctureTracker::InterpolateShift (:95-129), one CTA per tracker: its
+// threads look for the block that holds the puncture exclusively (MeshBlock::
+// PointContainedExclusive, mesh/meshblock.cpp:1186-1201; the first one), then
+// interpolate the shift there (LagrangeInterpND: x innermost, then y, then z),
+// a thread per x line, per y line, per component.  One thread searching 512
+// blocks took 494 us of every step.
+constexpr int kTrkThreads = 256;
+__global__ void __launch_bounds__(kTrkThreads)
+k_track_interp(Grid g, DevParams P, const double* __restrict__ u, double* __restrict__ trk) {
+  constexpr int n = kTrkOrder + 1;
+  __shared__ int owner, pt[3];
+  __shared__ double c[3][n], vy[3][n][n], vz[3][n];
+  double* T = trk + 8 * blockIdx.x;
   const int t = (int)threadIdx.x;
-  if (t >= ntrk) return;
-  double* T = trk + 8 * t;
   const double pos[3] = {T[0], T[1], T[2]};
   const int nsum = g.nn[0] + g.nn[1] + g.nn[2];
-  int owner = -1;
-  for (int b = 0; b < g.nblocks && owner < 0; ++b) {
+  if (t == 0) owner = g.nblocks;
+  __syncthreads();
+  for (int b = t; b < g.nblocks; b += kTrkThreads) {
     const double* x = P.xf + (int64_t)b * nsum;
     bool in = true;
     int off = 0;
+#pragma unroll
     for (int a = 0; a < 3; ++a) {
       in = in && (x[off + NG] <= pos[a]) && (pos[a] < x[off + NG + g.nx[a]]);
       off += g.nn[a];
     }
-    if (in) owner = b;
+    if (in) atomicMin(&owner, b);
   }
-  if (owner < 0) {  // the puncture has left the grid
-    T[6] = 1.0;
+  __syncthreads();
+  if (owner == g.nblocks) {  // the puncture has left the grid
+    if (t == 0) T[6] = 1.0;
     return;
   }
-  const double* x = P.xf + (int64_t)owner * nsum;
-  double c[3][kTrkOrder + 1];
-  int pt[3], off = 0;
-  for (int a = 0; a < 3; ++a) {
-    pt[a] = trk_lagrange1d(x[off], P.dx[(int64_t)owner * 3 + a], g.nn[a], pos[a], c[a]);
-    off += g.nn[a];
+  if (t < 3) {
+    int off = 0;
+    for (int a = 0; a < t; ++a) off += g.nn[a];
+    pt[t] = trk_lagrange1d(P.xf[(int64_t)owner * nsum + off], P.dx[(int64_t)owner * 3 + t],
+                           g.nn[t], pos[t], c[t]);
   }
-  for (int v = 0; v < 3; ++v) {
+  __syncthreads();
+  if (t < 3 * n * n) {
+    const int v = t / (n * n), ez = t / n % n, ey = t % n;
     const double* f = u + ((int64_t)owner * NVAR + Z4C_BETAX + v) * g.nvol;
-    double vz[kTrkOrder + 1];
-    for (int ez = 0; ez <= kTrkOrder; ++ez) {
-      double vy[kTrkOrder + 1];
-      for (int ey = 0; ey <= kTrkOrder; ++ey) {
-        const double* row = f + ((int64_t)(pt[2] + ez) * g.nn[1] + (pt[1] + ey)) * g.nn[0] + pt[0];
-        double o = 0;
-        for (int i = 0; i <= kTrkOrder; ++i) o += c[0][i] * row[i];
-        vy[ey] = o;
-      }
-      double o = 0;
-      for (int i = 0; i <= kTrkOrder; ++i) o += c[1][i] * vy[i];
-      vz[ez] = o;
-    }
+    const double* row = f + ((int64_t)(pt[2] + ez) * g.nn[1] + (pt[1] + ey)) * g.nn[0] + pt[0];
     double o = 0;
-    for (int i = 0; i <= kTrkOrder; ++i) o += c[2][i] * vz[i];
-    T[3 + v] = o;
+    for (int i = 0; i < n; ++i) o += c[0][i] * row[i];
+    vy[v][ez][ey] = o;
+  }
+  __syncthreads();
+  if (t < 3 * n) {
+    double o = 0;
+    for (int i = 0; i < n; ++i) o += c[1][i] * vy[t / n][t % n][i];
+    vz[t / n][t % n] = o;
+  }
+  __syncthreads();
+  if (t < 3) {
+    double o = 0;
+    for (int i = 0; i < n; ++i) o += c[2][i] * vz[t][i];
+    T[3 + t] = o;
   }
 }
 
@@ -1418,7 +1427,7 @@ static int upload_dir_index() {
 void launch_track_interp(const Grid& g, const DevParams& P, const double* u, double* trk,
                          int ntrk, cudaStream_t st) {
   COUNTED
-  k_track_interp<<<1, 32, 0, st>>>(g, P, u, trk, ntrk);
+  k_track_interp<<<ntrk, kTrkThreads, 0, st>>>(g, P, u, trk);
 }
 void launch_track_update(double* trk, int ntrk, double dt, cudaStream_t st) {
   COUNTED

@@ -257,28 +257,40 @@ uint64_t morton(const int loc[3]) {
 }
 
 // ---- kernels ----------------------------------------------------------------
-__global__ void k_wave_interp(Grid g, const double* __restrict__ weyl, const int* __restrict__ blk,
-                              const int* __restrict__ base, const double* __restrict__ coef,
-                              double* __restrict__ data, int npts) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= npts) return;
+// One CTA per vertex: a thread per x line of the two variables' 8^3 stencils,
+// then one per y line, one per variable; every sum in LagrangeInterpND::eval's
+// order (x innermost, then y, then z).  A thread per vertex walking its 1,024
+// values took 112 us for 1,002 vertices.
+__global__ void __launch_bounds__(2 * kSten * kSten)
+k_wave_interp(Grid g, const double* __restrict__ weyl, const int* __restrict__ blk,
+              const int* __restrict__ base, const double* __restrict__ coef,
+              double* __restrict__ data, int npts) {
+  __shared__ double vx[2][kSten][kSten], vy[2][kSten];
+  const int p = blockIdx.x, t = (int)threadIdx.x;
   const double* cf = coef + (int64_t)p * 3 * kSten;
-  for (int v = 0; v < 2; ++v) {
-    const double* f = weyl + ((int64_t)blk[p] * 2 + v) * g.nvol + base[p];
-    // LagrangeInterpND::eval: x innermost, then y, then z
-    double out = 0;
-    for (int ez = 0; ez < kSten; ++ez) {
-      double vy = 0;
-      for (int ey = 0; ey < kSten; ++ey) {
-        const double* row = f + ez * g.s[2] + ey * g.s[1];
-        double vx = 0;
+  {
+    const int v = t / (kSten * kSten), ez = t / kSten % kSten, ey = t % kSten;
+    const double* row =
+        weyl + ((int64_t)blk[p] * 2 + v) * g.nvol + base[p] + ez * g.s[2] + ey * g.s[1];
+    double o = 0;
 #pragma unroll
-        for (int i = 0; i < kSten; ++i) vx += cf[i] * __ldg(row + i);
-        vy += cf[kSten + ey] * vx;
-      }
-      out += cf[2 * kSten + ez] * vy;
-    }
-    data[(int64_t)v * npts + p] = out;
+    for (int i = 0; i < kSten; ++i) o += cf[i] * __ldg(row + i);
+    vx[v][ez][ey] = o;
+  }
+  __syncthreads();
+  if (t < 2 * kSten) {
+    const int v = t / kSten, ez = t % kSten;
+    double o = 0;
+#pragma unroll
+    for (int i = 0; i < kSten; ++i) o += cf[kSten + i] * vx[v][ez][i];
+    vy[v][ez] = o;
+  }
+  __syncthreads();
+  if (t < 2) {
+    double o = 0;
+#pragma unroll
+    for (int i = 0; i < kSten; ++i) o += cf[2 * kSten + i] * vy[t][i];
+    data[(int64_t)t * npts + p] = o;
   }
 }
 
@@ -293,7 +305,9 @@ __global__ void k_wave_project(const double* __restrict__ data, const double* __
   double pr = 0.0, pi = 0.0;
   if (mpl <= 2 * l) {
     const double* Y = ylm + (int64_t)slot * npts * 2;
-    for (int p = seg[sg]; p < seg[sg + 1]; ++p) {
+    const int end = seg[sg + 1];
+#pragma unroll 8  // eight vertices' loads in flight; the sums stay in order
+    for (int p = seg[sg]; p < end; ++p) {
       const double dr = data[p], di = data[npts + p];
       const double wt = pw[2 * p], bz = pw[2 * p + 1];
       const double yr = Y[2 * p], yi = Y[2 * p + 1];
@@ -452,10 +466,10 @@ void wave_free(WaveSphere* w) {
 
 void launch_wave(const Grid& g, const WaveSphere& w, const double* weyl, cudaStream_t st) {
   if (w.npts > 0) {
-    k_wave_interp<<<(w.npts + 127) / 128, 128, 0, st>>>(g, weyl, w.blk, w.base, w.coef, w.data,
+    k_wave_interp<<<w.npts, 2 * kSten * kSten, 0, st>>>(g, weyl, w.blk, w.base, w.coef, w.data,
                                                        w.npts);
     const int nt = w.nseg * w.nslot;
-    k_wave_project<<<(nt + 127) / 128, 128, 0, st>>>(w.data, w.pw, w.ylm, w.seg, w.loc, w.npts,
+    k_wave_project<<<(nt + 31) / 32, 32, 0, st>>>(w.data, w.pw, w.ylm, w.seg, w.loc, w.npts,
                                                      w.nseg, w.nslot, w.lmax);
     add_kernel_launches(2);
   }
@@ -465,7 +479,7 @@ void launch_wave(const Grid& g, const WaveSphere& w, const double* weyl, cudaStr
 
 void launch_wave_interp(const Grid& g, const WaveSphere& w, const double* weyl, cudaStream_t st) {
   if (w.npts <= 0) return;
-  k_wave_interp<<<(w.npts + 127) / 128, 128, 0, st>>>(g, weyl, w.blk, w.base, w.coef, w.data,
+  k_wave_interp<<<w.npts, 2 * kSten * kSten, 0, st>>>(g, weyl, w.blk, w.base, w.coef, w.data,
                                                      w.npts);
   add_kernel_launches(1);
 }
