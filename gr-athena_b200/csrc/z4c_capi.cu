@@ -588,7 +588,7 @@ int create_impl(const z4c_mesh_desc_t* mesh, const z4c_params_t* params, int int
     free_ctx(c);
     return fail(Z4C_ECUDA, "uploading mesh tables");
   }
-  if (allow_slab_smem() != 0) {
+  if (allow_slab_smem() != 0 || (c->ml && ml_prefer_l1() != 0)) {
     free_ctx(c);
     return fail(Z4C_ECUDA, "raising the shared-memory limit of the slab kernels");
   }

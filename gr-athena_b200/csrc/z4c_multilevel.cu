@@ -84,7 +84,12 @@ __device__ __forceinline__ int ml_zone(int i, int vs, int ve) {
 // coarse buffer (1).  The vertex's zone, multiplicity and contribution range
 // are found once and serve all nvar variables, whose loads are independent
 // of one another; the threads of a warp take consecutive vertices.
-__global__ void __launch_bounds__(kMlUnpackThreads)
+// kMlBatch variables at a time: a contribution's address is formed once for
+// them and their loads are in flight together (a variable at a time with 512
+// threads: 1.67 ms a fill on 512 blocks of 16^3, now 1.17, 4.0 GB).  grid z
+// cuts the vertices so that the last wave is short.
+constexpr int kMlBatch = 11, kMlGatherThreads = 256, kMlGatherParts = 4;
+__global__ void __launch_bounds__(kMlGatherThreads)
 k_ml_unpack(MlPlan P, const double* __restrict__ src, double* __restrict__ dst, int nvar,
             int reg_nvar) {
   const int b = blockIdx.x, arr = blockIdx.y;  // arr: 0 fine, 1 coarse
@@ -109,7 +114,7 @@ k_ml_unpack(MlPlan P, const double* __restrict__ src, double* __restrict__ dst, 
   const int64_t vs = vol;
   const double* own = arr ? P.csrc + (int64_t)b * Z4C_NVAR * vol : src + (int64_t)b * reg_nvar * vol;
   double* out = arr ? P.coarse + (int64_t)b * Z4C_NVAR * vol : dst + (int64_t)b * reg_nvar * vol;
-  for (int p = threadIdx.x; p < vol; p += blockDim.x) {
+  for (int p = blockIdx.z * blockDim.x + threadIdx.x; p < vol; p += gridDim.z * blockDim.x) {
     const int i = p % d0, row = p / d0, j = row % d1, k = row / d1;
     const int zi = ml_zone(i, ng, v0), zj = ml_zone(j, ng, v1), zk = ml_zone(k, ng, v2);
     const int z = (zk * 7 + zj) * 7 + zi;
@@ -117,20 +122,27 @@ k_ml_unpack(MlPlan P, const double* __restrict__ src, double* __restrict__ dst, 
     const int qb = zs[z] - c0, qe = zs[z + 1] - c0;
     const int m = mult[z];
     const double inv = m > 1 ? P.inv[m] : 1.0;
-#pragma unroll 2
-    for (int n = 0; n < nvar; ++n) {
-      double v = in ? __ldg(own + n * vs + p) : 0.0;
+    for (int n0 = 0; n0 < nvar; n0 += kMlBatch) {
+      const int nn = nvar - n0;
+      double v[kMlBatch];
+#pragma unroll
+      for (int n = 0; n < kMlBatch; ++n) v[n] = in && n < nn ? __ldg(own + (n0 + n) * vs + p) : 0.0;
       for (int q = qb; q < qe; ++q) {
         const MlContrib c = sc[q];
         const int64_t sv = c.scoarse ? P.cvol : P.fvol;
-        const double* s = c.scoarse ? P.csrc + ((int64_t)c.sblk * Z4C_NVAR + n) * sv
-                                    : src + ((int64_t)c.sblk * reg_nvar + n) * sv;
         const int s0 = c.scoarse ? P.cn[0] : P.nn[0], s1 = c.scoarse ? P.cn[1] : P.nn[1];
-        const double x = __ldg(s + ((k + c.d[2]) * s1 + j + c.d[1]) * s0 + i + c.d[0]);
-        v = c.mode == kMlCopy ? x : v + x;
+        const double* s = (c.scoarse ? P.csrc + ((int64_t)c.sblk * Z4C_NVAR + n0) * sv
+                                     : src + ((int64_t)c.sblk * reg_nvar + n0) * sv) +
+                          ((k + c.d[2]) * s1 + j + c.d[1]) * s0 + i + c.d[0];
+        double x[kMlBatch];
+#pragma unroll
+        for (int n = 0; n < kMlBatch; ++n) x[n] = n < nn ? __ldg(s + n * sv) : 0.0;
+#pragma unroll
+        for (int n = 0; n < kMlBatch; ++n) v[n] = c.mode == kMlCopy ? x[n] : v[n] + x[n];
       }
-      if (m > 1) v *= inv;
-      out[n * vs + p] = v;
+#pragma unroll
+      for (int n = 0; n < kMlBatch; ++n)
+        if (n < nn) out[(n0 + n) * vs + p] = m > 1 ? v[n] * inv : v[n];
     }
   }
 }
@@ -949,6 +961,19 @@ int ml_build(const int nroot[3], const int nx[3], const int bcf[6], int nblocks,
   return Z4C_OK;
 }
 
+int ml_prefer_l1() {
+  cudaError_t e = cudaSuccess;
+  auto prefer = [&](const void* k, int carveout) {
+    const cudaError_t r =
+        cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, carveout);
+    if (e == cudaSuccess) e = r;
+  };
+  prefer((const void*)k_ml_restrict, cudaSharedmemCarveoutMaxL1);
+  prefer((const void*)k_ml_unpack, 25);  // its tables and lists, a few kB per CTA
+  prefer((const void*)k_ml_prolong, cudaSharedmemCarveoutMaxL1);
+  return (int)e;
+}
+
 int launch_ml_exchange(const MlPlan& P, const double* src, double* dst, int nvar, int reg_nvar,
                        cudaStream_t st) {
   if (nvar < 1 || nvar > Z4C_NVAR || reg_nvar < nvar)
@@ -965,7 +990,8 @@ int launch_ml_exchange(const MlPlan& P, const double* src, double* dst, int nvar
       cudaFuncSetAttribute(k_ml_unpack, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)smem) != cudaSuccess)
     return set_error(Z4C_ECUDA, "multilevel exchange: shared memory for the contribution lists");
-  k_ml_unpack<<<dim3(P.nblocks, 2), kMlUnpackThreads, smem, st>>>(P, src, dst, nvar, reg_nvar);
+  k_ml_unpack<<<dim3(P.nblocks, 2, kMlGatherParts), kMlGatherThreads, smem, st>>>(
+      P, src, dst, nvar, reg_nvar);
   ++launches;
   auto bc_axis = [&](int lv, double* arr, int64_t bstride, int64_t vol, const int* dims, int ng) {
     for (int a = 0; a < 3; ++a) {

@@ -65,6 +65,10 @@ struct MlPlan {
                                      // from the coarse buffer (no other reads it)
 };
 
+// The fill's kernels read their neighbours through L1 and follow kernels that
+// leave little of it (see allow_slab_smem); returns a cudaError_t value.
+int ml_prefer_l1();
+
 // Builds the plan for nblocks MeshBlocks of nx cells given in gid order by
 // their logical locations locs[b] = {level, lx1, lx2, lx3} (absolute levels;
 // the root grid of nroot blocks per axis sits at the level whose 2^level
