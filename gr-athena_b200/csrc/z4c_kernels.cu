@@ -1248,33 +1248,17 @@ bool slabs_fit(const Grid& g, const LaunchShape& sh) {
   size_t b;
   return slab_geom(g, sh, &b).kper > 0;
 }
-// Lets every slab kernel take up to kSlabMaxBytes of dynamic shared memory.
-// Runs before any launch (at context creation), never inside a captured
-// stream.
-int allow_slab_smem() {
+// The other kernels of a step read their neighbours through L1, and follow
+// kernels whose shared memory leaves little of it: without the preference the
+// split stays as those left it (three evolutions of 512 blocks of 16^3 on
+// three streams: 23.4 ms a step against 19.5).  A hint, given once per device.
+static cudaError_t prefer_l1() {
+  static std::atomic<unsigned long long> given{0};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return cudaGetLastError();
+  const unsigned long long bit = 1ull << (dev & 63);
+  if (given.load() & bit) return cudaSuccess;
   cudaError_t e = cudaSuccess;
-  auto set = [&](const void* k) {
-    const cudaError_t r =
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSlabMaxBytes);
-    if (e == cudaSuccess) e = r;
-  };
-  set((const void*)k_ko_rhs_slab);
-  set((const void*)k_ko_stage_ls_slab<true>);
-  set((const void*)k_ko_stage_ls_slab<false>);
-  set((const void*)k_ko_stage_bt_slab<true>);
-  set((const void*)k_ko_stage_bt_slab<false>);
-  auto raise = [&](const void* k, int bytes) {
-    const cudaError_t r =
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess) e = r;
-  };
-  raise((const void*)k_deriv<false, 18, 17>, kDvMaxSmem);
-  raise((const void*)k_deriv<false, 34, 9>, kDvMaxSmem);
-  raise((const void*)k_point, kStageBytes);
-  // The other kernels of a step read their neighbours through L1, and follow
-  // kernels whose shared memory leaves little of it: without the preference
-  // the split stays as those left it (three evolutions of 512 blocks of 16^3
-  // on three streams: 23.4 ms a step against 19.5).
   constexpr int F = kFixedNX, M = kMergedNX, U = kColUnroll;
   for (const void* k :
        {(const void*)k_ko_stage_ls<F + 1, true, true, F>, (const void*)k_ko_stage_ls<F + 1, true, false, F>,
@@ -1302,6 +1286,34 @@ int allow_slab_smem() {
                                                cudaSharedmemCarveoutMaxL1);
     if (e == cudaSuccess) e = r;
   }
+  if (e == cudaSuccess) given.fetch_or(bit);
+  return e;
+}
+
+// Lets every slab kernel take up to kSlabMaxBytes of dynamic shared memory.
+// Runs before any launch (at context creation), never inside a captured
+// stream.
+int allow_slab_smem() {
+  cudaError_t e = cudaSuccess;
+  auto set = [&](const void* k) {
+    const cudaError_t r =
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSlabMaxBytes);
+    if (e == cudaSuccess) e = r;
+  };
+  set((const void*)k_ko_rhs_slab);
+  set((const void*)k_ko_stage_ls_slab<true>);
+  set((const void*)k_ko_stage_ls_slab<false>);
+  set((const void*)k_ko_stage_bt_slab<true>);
+  set((const void*)k_ko_stage_bt_slab<false>);
+  auto raise = [&](const void* k, int bytes) {
+    const cudaError_t r =
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) e = r;
+  };
+  raise((const void*)k_deriv<false, 18, 17>, kDvMaxSmem);
+  raise((const void*)k_deriv<false, 34, 9>, kDvMaxSmem);
+  raise((const void*)k_point, kStageBytes);
+  if (e == cudaSuccess) e = prefer_l1();
   if (e == cudaSuccess) e = (cudaError_t)allow_deriv_smem_fast();
   return (int)e;
 }

@@ -30,6 +30,8 @@
 // [block][var][cn3][cn2][cn1] with cn = nx/2 + 1 + 2 NCG.
 #include <cuda_runtime.h>
 
+#include <atomic>
+
 #include <algorithm>
 #include <cstdint>
 #include <cstring>
@@ -961,8 +963,12 @@ int ml_build(const int nroot[3], const int nx[3], const int bcf[6], int nblocks,
   return Z4C_OK;
 }
 
-int ml_prefer_l1() {
-  cudaError_t e = cudaSuccess;
+int ml_prefer_l1() {  // a hint, given once per device
+  static std::atomic<unsigned long long> given{0};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  const unsigned long long bit = 1ull << (dev & 63);
+  if (e != cudaSuccess || (given.load() & bit)) return (int)e;
   auto prefer = [&](const void* k, int carveout) {
     const cudaError_t r =
         cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, carveout);
@@ -971,6 +977,7 @@ int ml_prefer_l1() {
   prefer((const void*)k_ml_restrict, cudaSharedmemCarveoutMaxL1);
   prefer((const void*)k_ml_unpack, 25);  // its tables and lists, a few kB per CTA
   prefer((const void*)k_ml_prolong, cudaSharedmemCarveoutMaxL1);
+  if (e == cudaSuccess) given.fetch_or(bit);
   return (int)e;
 }
 
