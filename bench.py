@@ -89,8 +89,9 @@ FP64_OPS_PER_POINT_STAGE = 7697 + 154
 # The launches of one fused stage and their measured DRAM traffic per interior
 # vertex (ncu dram__bytes_read.sum + dram__bytes_write.sum summed over them,
 # 64-block capture scaled by the vertex count; see profiles/).
-STAGE_KERNELS = {0: "k_prep, k_ricci, k_adv, k_main, k_ko_stage_ls",
-                 1: "k_prep, k_ricci_fast, k_main_fast, k_col_fast"}
+STAGE_KERNELS = {0: "k_deriv, k_point, k_ko_stage_ls",
+                 1: "k_deriv, k_point_fast; on the 128^3 merged grid k_prep, "
+                    "k_stencil_point, k_col_fast"}
 # FP64 operations of PrepareZ4cDerivatives + Z4cWeyl per interior vertex
 # (oracle/opcount), for the psi4 diagnostics line.
 FP64_OPS_PER_POINT_WEYL = 7409
