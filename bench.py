@@ -87,8 +87,8 @@ STAGE_BYTES_PER_POINT = 4 * 22 * 8
 # for the low-storage stage update (7 per variable).
 FP64_OPS_PER_POINT_STAGE = 7697 + 154
 # The launches of one fused stage and their measured DRAM traffic per interior
-# vertex (ncu dram__bytes_read.sum + dram__bytes_write.sum summed over them,
-# 64-block capture scaled by the vertex count; see profiles/).
+# vertex (ncu dram__bytes_read.sum + dram__bytes_write.sum summed over them on
+# the 512 blocks; not captured for the merged grid's stage).
 STAGE_KERNELS = {0: "k_deriv, k_point, k_ko_stage_ls",
                  1: "k_deriv, k_point_fast; on the 128^3 merged grid k_prep, "
                     "k_stencil_point, k_col_fast"}
@@ -98,10 +98,7 @@ FP64_OPS_PER_POINT_WEYL = 7409
 # psi4 extraction spheres of the diagnostics: (radius, nlev, lmax) inside
 # the [-16,16]^3 domain
 WAVE_SPHERES = ((6.0, 30, 8), (12.0, 30, 8))
-STAGE_TRAFFIC_PER_POINT = {0: 1350.0e6 / (64 * 17 ** 3), 1: 1025.6e6 / (64 * 17 ** 3),
-                           # the contracted stage on a merged grid: ncu on the 97^3-vertex
-                           # grid of 6^3 blocks (registers 204 MB), per vertex
-                           "merged": 2153.4e6 / 97 ** 3}
+STAGE_TRAFFIC_PER_POINT = {0: 11764.0e6 / (512 * 17 ** 3), 1: 9193.0e6 / (512 * 17 ** 3)}
 
 
 def parse():
