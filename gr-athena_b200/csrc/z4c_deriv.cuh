@@ -9,13 +9,12 @@
 
 #include "z4c_common.cuh"
 #include "z4c_kernels.cuh"
+#include "z4c_pieces.h"
 #include "z4c_stencil.cuh"
 
 namespace z4c {
 
-// Layout of the scratch: [block][group of 32 interior vertices of the slab]
-// [component][vertex of the group], so that a warp of the pointwise pass finds
-// all of its operands in one contiguous piece.
+// Components of a vertex in the scratch (its layout: z4c_pieces.h).
 // The variables with second derivatives (chi, g~, alpha, beta: slot s) take
 // nine components each, D_x D_y D_z and D_xx D_xy D_xz D_yy D_yz D_zz; Khat,
 // Gamma~ and Theta three; every variable one advection sum (contracted path:
@@ -25,9 +24,8 @@ constexpr int kDvGrad = 5;                      // with first derivatives only
 constexpr int kDvFirst = 9 * kDvHess;           // first component of the latter
 constexpr int kDvAdv = kDvFirst + 3 * kDvGrad;  // first advection sum
 constexpr int kDvComponents = kDvAdv + NVAR;
-constexpr int kDvGroup = 32;
 __host__ __device__ __forceinline__ constexpr int64_t dv_doubles(int64_t vertices) {
-  return (vertices + kDvGroup - 1) / kDvGroup * kDvGroup * kDvComponents;
+  return dv_doubles(vertices, kDvComponents);
 }
 
 // Variable of the f-th CTA row: the slots with second derivatives first (the
@@ -405,26 +403,10 @@ inline DerivLaunch deriv_launch(const Grid& g, int nblk, int ks, int nk) {
   return L;
 }
 
-// Runs the derivative and pointwise passes on nblk blocks in pieces whose
-// scratch fits: all at once, by equal groups of blocks, or, where one block
-// does not fit, by slabs of planes of each block.  launch(b, nb, ks, nk) takes
-// blocks b .. b + nb - 1 and interior planes ks .. ks + nk - 1.
+// for_deriv_chunks on the passes' scratch.
 template <class Launch>
 inline void for_deriv_chunks(const Grid& g, int nblk, const RhsScratch& sc, Launch launch) {
-  const int nk = g.nx[2] + 1;
-  const int64_t plane = (int64_t)(g.nx[0] + 1) * (g.nx[1] + 1);
-  const int64_t per = dv_doubles(plane * nk);
-  if (per <= sc.cap) {
-    const int64_t pieces = (nblk * per + sc.cap - 1) / sc.cap;
-    const int nb = (int)((nblk + pieces - 1) / pieces);
-    for (int b = 0; b < nblk; b += nb) launch(b, nblk - b < nb ? nblk - b : nb, 0, nk);
-    return;
-  }
-  const int64_t most = (sc.cap / kDvComponents - kDvGroup) / plane;  // planes that fit
-  const int64_t slabs = (nk + most - 1) / most;
-  const int h = (int)((nk + slabs - 1) / slabs);
-  for (int b = 0; b < nblk; ++b)
-    for (int k = 0; k < nk; k += h) launch(b, 1, k, nk - k < h ? nk - k : h);
+  for_deriv_chunks(g.nx, nblk, kDvComponents, sc.cap, launch);
 }
 
 }  // namespace z4c
