@@ -18,6 +18,7 @@
 #include "z4c_common.cuh"
 #include "z4c_kernels.cuh"
 #include "z4c_multilevel.cuh"
+#include "z4c_pieces.h"
 #include "z4c_restart.cuh"
 #include "z4c_wave.cuh"
 #include "z4c_ctx.cuh"
@@ -260,7 +261,7 @@ int run_stage_body(z4c_ctx* c, int stage, double dt) {
     const double w1[3] = {1.0, wt[0], 0.0};
     const double w2[3] = {wt[1], wt[2], wt[3]};
     for (int b = 0; b < g.nblocks; ++b) {
-      launch_rhs(g, P, u, c->scratch(), c->reg[Z4C_REG_RHS], b, 1, c->shape, c->stream);
+      launch_rhs(g, P, u, c->scratch(b, 1), c->reg[Z4C_REG_RHS], b, 1, c->shape, c->stream);
       launch_boundary_rhs(g, P, u, c->reg[Z4C_REG_RHS], b, 1, c->stream);
       launch_weighted_ave(g, c->reg[Z4C_REG_U1], u, nullptr, w1, b, 1, c->stream);
       launch_weighted_ave(g, u, c->reg[Z4C_REG_U1], nullptr, w2, b, 1, c->stream);
@@ -300,7 +301,7 @@ int run_stage_body(z4c_ctx* c, int stage, double dt) {
     return exchange_into(c, w, u, true);
   }
   for (int b = 0; b < g.nblocks; ++b) {
-    launch_stage_bt(g, P, u, c->scratch(), c->reg[Z4C_REG_RHS], c->un, K, w, bs, b, 1,
+    launch_stage_bt(g, P, u, c->scratch(b, 1), c->reg[Z4C_REG_RHS], c->un, K, w, bs, b, 1,
                     c->shape, c->stream);
     LAUNCH_CHECK("stage_bt");
   }
@@ -554,18 +555,14 @@ int create_impl(const z4c_mesh_desc_t* mesh, const z4c_params_t* params, int int
   if (rc == Z4C_OK && integrator == Z4C_INTEG_BT_RK4) rc = alloc((void**)&c->un, b22);
   if (rc == Z4C_OK) rc = alloc((void**)&c->guu, sizeof(double) * 6 * (size_t)g.nvol * nb);
   {
-    // The right-hand-side scratch: the diagnostics' and the adjoint's three
-    // arrays, or the derivative pass's components of every interior vertex
-    // where that is at most a little more or small in itself (otherwise the
-    // passes run in pieces that fit).
-    const int64_t npts = interior_count(g), first = (int64_t)kSdComponents * g.nvol * nb;
-    const int64_t parts = first + 28 * npts * nb, whole = rhs_scratch_doubles(g) * nb;
-    c->scratch_cap = whole <= parts + parts / 16 || whole <= (int64_t)1 << 29
-                         ? std::max(parts, whole) : parts;
-    if (rc == Z4C_OK) rc = alloc((void**)&c->sd, sizeof(double) * (size_t)c->scratch_cap);
+    const int64_t npts = interior_count(g);
+    c->scratch_share = dv_context_share((int64_t)kSdComponents * g.nvol + 28 * npts,
+                                        rhs_scratch_doubles(g), nb);
+    if (rc == Z4C_OK)
+      rc = alloc((void**)&c->sd, sizeof(double) * (size_t)c->scratch_share * nb);
     if (rc == Z4C_OK) {
-      c->rsum = c->sd + first;
-      c->lv = c->rsum + 6 * npts * nb;
+      c->rsum = c->scratch().rsum;
+      c->lv = c->scratch().lv;
     }
   }
   if (rc == Z4C_OK) rc = alloc((void**)&c->xf, sizeof(double) * c->h_xf.size());
@@ -767,7 +764,7 @@ int z4c_rhs(z4c_ctx* ctx, int reg_u, int reg_rhs, int block) {
   if (reg_nvar_(reg_u) != Z4C_NVAR || reg_nvar_(reg_rhs) != Z4C_NVAR || reg_u == reg_rhs)
     return fail(Z4C_EINVAL, "z4c_rhs needs two distinct 22-variable registers");
   if ((rc = check_block(ctx, block, &b0, &nb))) return rc;
-  launch_rhs(ctx->g, ctx->dev(), ctx->reg[reg_u], ctx->scratch(), ctx->reg[reg_rhs], b0, nb,
+  launch_rhs(ctx->g, ctx->dev(), ctx->reg[reg_u], ctx->scratch(b0, nb), ctx->reg[reg_rhs], b0, nb,
              ctx->shape, ctx->stream);
   LAUNCH_CHECK("rhs");
   return Z4C_OK;
@@ -859,7 +856,7 @@ int z4c_adm_constraints(z4c_ctx* ctx, int reg_con, int reg_adm, int reg_u, int b
       reg_nvar_(reg_u) != Z4C_NVAR)
     return fail(Z4C_EINVAL, "ADMConstraints needs con, adm and a Z4c register");
   if ((rc = check_block(ctx, block, &b0, &nb))) return rc;
-  CUDA_TRY((cudaError_t)launch_adm_constraints(ctx->g, ctx->dev(), ctx->scratch(),
+  CUDA_TRY((cudaError_t)launch_adm_constraints(ctx->g, ctx->dev(), ctx->scratch(b0, nb),
                                                ctx->reg[reg_adm], ctx->reg[reg_u],
                                                ctx->reg[reg_con], ctx->xf, b0, nb, ctx->stream));
   return Z4C_OK;
@@ -875,7 +872,8 @@ int z4c_weyl(z4c_ctx* ctx, int reg_adm, int reg_u, int reg_weyl, int block) {
       reg_nvar_(reg_weyl) != Z4C_NWEYL)
     return fail(Z4C_EINVAL, "Z4cWeyl needs the ADM, a Z4c and the Weyl register");
   if ((rc = check_block(ctx, block, &b0, &nb))) return rc;
-  launch_weyl(ctx->g, ctx->dev(), ctx->reg[reg_adm], ctx->reg[reg_u], ctx->sd, ctx->rsum, ctx->lv,
+  const RhsScratch sc = ctx->scratch(b0, nb);
+  launch_weyl(ctx->g, ctx->dev(), ctx->reg[reg_adm], ctx->reg[reg_u], sc.sd, sc.rsum, sc.lv,
               ctx->reg[reg_weyl], ctx->xf, b0, nb, ctx->stream);
   LAUNCH_CHECK("weyl");
   return Z4C_OK;

@@ -62,11 +62,11 @@ struct z4c_ctx {
   double* reg[Z4C_NREG] = {};
   double* un = nullptr;   // Butcher u_n scratch
   double* guu = nullptr;  // ADMToZ4c inverse-metric scratch (6 vars)
-  double* sd = nullptr;   // right-hand-side scratch; its parts when used as such:
-                          // stored first derivatives, 33 values per vertex,
-  double* rsum = nullptr; // then Ricci sums, 6 values per interior vertex,
-  double* lv = nullptr;   // then 22 values per interior vertex
-  int64_t scratch_cap = 0;  // doubles at sd
+  double* sd = nullptr;   // right-hand-side scratch; its parts when used as such
+                          // on every block: stored first derivatives, 33 values
+  double* rsum = nullptr; // per vertex, then Ricci sums, 6 values per interior
+  double* lv = nullptr;   // vertex, then 22 values per interior vertex
+  int64_t scratch_share = 0;  // doubles of each block's share at sd
   double* xf = nullptr;   // [nblocks][nn0+nn1+nn2]
   double* xv = nullptr;   // [nblocks][nn0+nn1+nn2-3]
   double* dxd = nullptr;  // [nblocks][3] vertex spacing
@@ -100,7 +100,15 @@ struct z4c_ctx {
   double graph_dt = 0.0;
   bool graph_per_block = false;
 
-  RhsScratch scratch() const { return RhsScratch{sd, rsum, lv, sd, scratch_cap}; }
+  RhsScratch scratch() const { return scratch(0, g.nblocks); }
+  // For a call on blocks b .. b + nb - 1: the parts, indexed by absolute block,
+  // lie one behind the other in these blocks' shares.
+  RhsScratch scratch(int b, int nb) const {
+    const int64_t np = interior_count(g), first = (int64_t)kSdComponents * g.nvol;
+    double* const at = sd + b * scratch_share;
+    return RhsScratch{at - b * first, at + nb * first - b * 6 * np,
+                      at + nb * (first + 6 * np) - b * 22 * np, sd, scratch_share};
+  }
 
   DevParams dev() const {
     DevParams P;

@@ -403,10 +403,14 @@ inline DerivLaunch deriv_launch(const Grid& g, int nblk, int ks, int nk) {
   return L;
 }
 
-// for_deriv_chunks on the passes' scratch.
+// for_deriv_chunks on the passes' scratch: launch(b, nb, ks, nk, scratch).
 template <class Launch>
-inline void for_deriv_chunks(const Grid& g, int nblk, const RhsScratch& sc, Launch launch) {
-  for_deriv_chunks(g.nx, nblk, kDvComponents, sc.cap, launch);
+inline void for_deriv_chunks(const Grid& g, int block0, int nblk, const RhsScratch& sc,
+                             Launch launch) {
+  for_deriv_chunks(g.nx, block0, nblk, kDvComponents, sc.share,
+                   [&](int b, int nb, int ks, int nk, int64_t at) {
+                     launch(b, nb, ks, nk, sc.base + at);
+                   });
 }
 
 }  // namespace z4c

@@ -163,13 +163,13 @@ void launch_fast(const Grid& g, const DevParams& P, const double* u, const RhsSc
     launch_merged<STAGE>(g, P, u, sc, rhs, u1, u_out, w, block0, nblk, st);
     return;
   }
-  for_deriv_chunks(g, nblk, sc, [&](int b, int nb, int ks, int nk) {
+  for_deriv_chunks(g, block0, nblk, sc, [&](int b, int nb, int ks, int nk, double* D) {
     const DerivLaunch L = deriv_launch(g, nb, ks, nk);
     (L.narrow ? k_deriv<true, 18, 17> : k_deriv<true, 34, 9>)<<<L.grid, L.threads, L.smem, st>>>(
-        g, P, u, sc.base, L.T, block0 + b);
+        g, P, u, D, L.T, b);
     const int64_t np = (int64_t)nk * (g.nx[1] + 1) * (g.nx[0] + 1);
     k_point_fast<STAGE><<<dim3(div_up(np, kDvGroup), nb), kDvGroup, kStageBytes, st>>>(
-        g, P, u, sc.base, rhs, u1, u_out, w, block0 + b, ks, nk);
+        g, P, u, D, rhs, u1, u_out, w, b, ks, nk);
     add_kernel_launches(2);
   });
 }

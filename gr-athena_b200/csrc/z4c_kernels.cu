@@ -1323,16 +1323,15 @@ int allow_slab_smem() {
 static void launch_rhs_passes(const Grid& g, const DevParams& P, const double* u,
                               const RhsScratch& sc, double* rhs, int block0, int nblk,
                               cudaStream_t st) {
-  for_deriv_chunks(g, nblk, sc, [&](int b, int nb, int ks, int nk) {
+  for_deriv_chunks(g, block0, nblk, sc, [&](int b, int nb, int ks, int nk, double* D) {
     const DerivLaunch L = deriv_launch(g, nb, ks, nk);
     COUNTED
     (L.narrow ? k_deriv<false, 18, 17> : k_deriv<false, 34, 9>)<<<L.grid, L.threads, L.smem,
-                                                                  st>>>(g, P, u, sc.base, L.T,
-                                                                        block0 + b);
+                                                                  st>>>(g, P, u, D, L.T, b);
     const int64_t np = (int64_t)nk * (g.nx[1] + 1) * (g.nx[0] + 1);
     COUNTED
     k_point<<<dim3(div_up(np, kDvGroup), nb), kDvGroup, kStageBytes, st>>>(
-        g, P, u, sc.base, rhs, block0 + b, ks, nk);
+        g, P, u, D, rhs, b, ks, nk);
   });
 }
 
@@ -1581,17 +1580,16 @@ int launch_adm_constraints(const Grid& g, const DevParams& P, const RhsScratch& 
       cudaMemsetAsync(con + (int64_t)block0 * Z4C_NCON * g.nvol, 0,
                       sizeof(double) * (size_t)Z4C_NCON * g.nvol * nblk, st);
   if (e != cudaSuccess) return (int)e;
-  for_deriv_chunks(g, nblk, sc, [&](int b, int nb, int ks, int nk) {
+  for_deriv_chunks(g, block0, nblk, sc, [&](int b, int nb, int ks, int nk, double* D) {
     DerivLaunch L = deriv_launch(g, nb, ks, nk);
     L.grid.y = kConComponents / 9;
     COUNTED
     (L.narrow ? k_deriv<false, 18, 17> : k_deriv<false, 34, 9>)<<<L.grid, L.threads, L.smem,
-                                                                  st>>>(g, P, u, sc.base, L.T,
-                                                                        block0 + b);
+                                                                  st>>>(g, P, u, D, L.T, b);
     const int64_t np = (int64_t)nk * (g.nx[1] + 1) * (g.nx[0] + 1);
     COUNTED
     k_adm_constraints<<<dim3(div_up(np, kDvGroup), nb), kDvGroup, 0, st>>>(
-        g, P, adm, u, sc.base, con, xf, block0 + b, ks, nk);
+        g, P, adm, u, D, con, xf, b, ks, nk);
   });
   return (int)cudaGetLastError();
 }

@@ -52,10 +52,11 @@ long long kernel_launch_count();
 void add_kernel_launches(long long n);
 
 // All launches return cudaGetLastError() mapped by the caller.
-// Scratch of the right-hand-side passes: base, cap doubles, holds what the
-// derivative pass leaves for the pointwise pass (z4c_deriv.cuh), in pieces
-// where it does not hold the whole mesh.  The diagnostics and the adjoint use
-// the same memory, by absolute block, as sd [block][33][vertex] (stored first
+// Scratch of the right-hand-side passes: base, share doubles for each block of
+// the mesh in turn, holds what the derivative pass leaves for the pointwise
+// pass (z4c_deriv.cuh), in pieces where it does not hold every component.  A
+// call on some blocks uses their shares only.  The diagnostics and the adjoint
+// use these shares, by absolute block, as sd [block][33][vertex] (stored first
 // derivatives of chi, g~, alpha, beta along x, y, z), rsum [block][6][interior
 // vertex] (R_ab + Rphi_ab) and lv [block][22][interior vertex].
 struct RhsScratch {
@@ -63,7 +64,7 @@ struct RhsScratch {
   double* rsum;
   double* lv;
   double* base;
-  int64_t cap;
+  int64_t share;
 };
 constexpr int kSdComponents = 33;
 // Scratch doubles per block of the derivative pass.

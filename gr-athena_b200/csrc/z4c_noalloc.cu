@@ -33,6 +33,7 @@
 #include "../../include/z4c_b200.h"
 #include "z4c_common.cuh"
 #include "z4c_kernels.cuh"
+#include "z4c_pieces.h"
 
 namespace z4c {
 int set_error(int code, const char* msg);
@@ -152,12 +153,8 @@ extern "C" int z4c_rhs_noalloc(const double* u, double* rhs, int nblocks, const 
   int rc = scratch_for_current_device(&base);
   if (rc) return rc;
   FdScale* fd = reinterpret_cast<FdScale*>(base);
-  RhsScratch sc;
-  sc.sd = base + kFdBytes / sizeof(double);
-  sc.rsum = sc.sd + (size_t)kSdComponents * g.nvol * chunk;
-  sc.lv = sc.rsum + (size_t)6 * npts * chunk;
-  sc.base = sc.sd;
-  sc.cap = (int64_t)(room / sizeof(double));
+  RhsScratch sc{};
+  sc.base = base + kFdBytes / sizeof(double);
 
   // FD scalings of finite_differencing.tpp:20-56, as z4c_create computes them
   FdScale f;
@@ -183,6 +180,7 @@ extern "C" int z4c_rhs_noalloc(const double* u, double* rhs, int nblocks, const 
     g.nb[0] = nb;
     g.nb[1] = g.nb[2] = 1;
     g.nblocks = nb;
+    sc.share = dv_share((int64_t)(room / sizeof(double)), nb);
     launch_rhs(g, P, u + bstride * b0, sc, rhs + bstride * b0, 0, nb, LaunchShape(), st);
   }
   const cudaError_t e = cudaGetLastError();

@@ -21,14 +21,32 @@ Z4C_PIECES_HD constexpr int64_t dv_doubles(int64_t vertices, int components) {
   return (vertices + kDvGroup - 1) / kDvGroup * kDvGroup * components;
 }
 
-// Runs the derivative and pointwise passes on nblk blocks of nx cells in pieces
-// whose scratch fits cap doubles: all at once, by equal groups of blocks, or,
-// where one block does not fit, by slabs of planes of each block.
-// launch(b, nb, ks, nk) takes blocks b .. b + nb - 1 and interior planes ks ..
-// ks + nk - 1.
+// Every block of the mesh has its share of the scratch, and a call uses the
+// shares of its own blocks only, so that calls on different blocks may run at
+// the same time on different streams.  Shares are whole groups: they start on
+// 256-byte boundaries.
+inline int64_t dv_share(int64_t cap, int nblocks) {
+  return cap / nblocks / kDvGroup * kDvGroup;
+}
+// A context's share of a block: what the diagnostics and the adjoint need
+// (parts), or every component of the derivative pass (whole) where that is at
+// most a little more, or small on the mesh (512 Mi doubles); otherwise the
+// passes run in pieces that fit.
+inline int64_t dv_context_share(int64_t parts, int64_t whole, int nblocks) {
+  parts = (parts + kDvGroup - 1) / kDvGroup * kDvGroup;
+  const bool all = whole <= parts + parts / 16 || whole * nblocks <= (int64_t)1 << 29;
+  return all && whole > parts ? whole : parts;
+}
+
+// Runs the derivative and pointwise passes on blocks block0 .. block0 + nblk - 1
+// of nx cells in pieces whose scratch fits these blocks' shares: all at once,
+// by equal groups of blocks, or, where one block does not fit, by slabs of
+// planes of each block.  launch(b, nb, ks, nk, at) takes blocks b .. b + nb - 1
+// and interior planes ks .. ks + nk - 1, with its scratch at double `at`.
 template <class Launch>
-inline void for_deriv_chunks(const int nx[3], int nblk, int components, int64_t cap,
+inline void for_deriv_chunks(const int nx[3], int block0, int nblk, int components, int64_t share,
                              Launch launch) {
+  const int64_t at = block0 * share, cap = nblk * share;
   const int nk = nx[2] + 1;
   const int64_t plane = (int64_t)(nx[0] + 1) * (nx[1] + 1);
   const int64_t per = dv_doubles(plane * nk, components);
@@ -36,14 +54,15 @@ inline void for_deriv_chunks(const int nx[3], int nblk, int components, int64_t 
     const int64_t room = cap / per;  // blocks that fit
     const int64_t pieces = (nblk + room - 1) / room;
     const int nb = (int)((nblk + pieces - 1) / pieces);
-    for (int b = 0; b < nblk; b += nb) launch(b, nblk - b < nb ? nblk - b : nb, 0, nk);
+    for (int b = 0; b < nblk; b += nb)
+      launch(block0 + b, nblk - b < nb ? nblk - b : nb, 0, nk, at);
     return;
   }
   const int64_t most = (cap / components - kDvGroup) / plane;  // planes that fit
   const int64_t slabs = (nk + most - 1) / most;
   const int h = (int)((nk + slabs - 1) / slabs);
   for (int b = 0; b < nblk; ++b)
-    for (int k = 0; k < nk; k += h) launch(b, 1, k, nk - k < h ? nk - k : h);
+    for (int k = 0; k < nk; k += h) launch(block0 + b, 1, k, nk - k < h ? nk - k : h, at);
 }
 
 }  // namespace z4c
