@@ -320,7 +320,7 @@ void free_ctx(z4c_ctx* c) {
   c->reg[Z4C_REG_TAN] = c->reg[Z4C_REG_ADJ] = c->reg[Z4C_REG_ADM_ADJ] = nullptr;
   for (auto& r : c->reg)
     if (r) cudaFree(r);
-  for (void* p : {(void*)c->un, (void*)c->guu, (void*)c->sd, (void*)c->xf, (void*)c->xv, (void*)c->dxd, (void*)c->fd,
+  for (void* p : {(void*)c->un, (void*)c->guu, (void*)c->sd, (void*)c->con.base, (void*)c->xf, (void*)c->xv, (void*)c->dxd, (void*)c->fd,
                   (void*)c->nbr, (void*)c->partials, (void*)c->flag, (void*)c->trk})
     if (p) cudaFree(p);
   for (auto& w : c->waves) wave_free(&w);
@@ -564,6 +564,9 @@ int create_impl(const z4c_mesh_desc_t* mesh, const z4c_params_t* params, int int
       c->rsum = c->scratch().rsum;
       c->lv = c->scratch().lv;
     }
+    c->con.share = con_scratch_share(g);
+    if (rc == Z4C_OK)
+      rc = alloc((void**)&c->con.base, sizeof(double) * (size_t)c->con.share * nb);
   }
   if (rc == Z4C_OK) rc = alloc((void**)&c->xf, sizeof(double) * c->h_xf.size());
   if (rc == Z4C_OK) rc = alloc((void**)&c->xv, sizeof(double) * c->h_xv.size());
@@ -856,7 +859,7 @@ int z4c_adm_constraints(z4c_ctx* ctx, int reg_con, int reg_adm, int reg_u, int b
       reg_nvar_(reg_u) != Z4C_NVAR)
     return fail(Z4C_EINVAL, "ADMConstraints needs con, adm and a Z4c register");
   if ((rc = check_block(ctx, block, &b0, &nb))) return rc;
-  CUDA_TRY((cudaError_t)launch_adm_constraints(ctx->g, ctx->dev(), ctx->scratch(b0, nb),
+  CUDA_TRY((cudaError_t)launch_adm_constraints(ctx->g, ctx->dev(), ctx->con,
                                                ctx->reg[reg_adm], ctx->reg[reg_u],
                                                ctx->reg[reg_con], ctx->xf, b0, nb, ctx->stream));
   return Z4C_OK;
@@ -1429,7 +1432,7 @@ int merged_evolve(z4c_ctx* c, double dt, int nsteps, int with_constraints) {
   LAUNCH_CHECK("z4c_to_adm");
   if (with_constraints) {
     CUDA_TRY((cudaError_t)launch_adm_constraints(
-        c->g, P, c->scratch(), c->reg[Z4C_REG_ADM], c->reg[Z4C_REG_U], c->reg[Z4C_REG_CON], c->xf,
+        c->g, P, c->con, c->reg[Z4C_REG_ADM], c->reg[Z4C_REG_U], c->reg[Z4C_REG_CON], c->xf,
         0, c->g.nblocks, c->stream));
   }
   if (c->ntrk > 0)
@@ -1486,7 +1489,7 @@ int z4c_evolve(z4c_ctx* ctx, double dt, int nsteps, int with_constraints) {
       launch_z4c_to_adm(ctx->g, P, ctx->reg[Z4C_REG_U], ctx->reg[Z4C_REG_ADM], 0, ctx->g.nblocks,
                         ctx->stream);
     CUDA_TRY((cudaError_t)launch_adm_constraints(
-        ctx->g, P, ctx->scratch(), ctx->reg[Z4C_REG_ADM], ctx->reg[Z4C_REG_U],
+        ctx->g, P, ctx->con, ctx->reg[Z4C_REG_ADM], ctx->reg[Z4C_REG_U],
         ctx->reg[Z4C_REG_CON], ctx->xf, 0, ctx->g.nblocks, ctx->stream));
   }
   return Z4C_OK;

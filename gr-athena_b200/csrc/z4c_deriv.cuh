@@ -24,6 +24,7 @@ constexpr int kDvGrad = 5;                      // with first derivatives only
 constexpr int kDvFirst = 9 * kDvHess;           // first component of the latter
 constexpr int kDvAdv = kDvFirst + 3 * kDvGrad;  // first advection sum
 constexpr int kDvComponents = kDvAdv + NVAR;
+constexpr int kDvCon = 9 * 7;  // the constraints' components: chi and g~
 __host__ __device__ __forceinline__ constexpr int64_t dv_doubles(int64_t vertices) {
   return dv_doubles(vertices, kDvComponents);
 }
@@ -134,8 +135,9 @@ __device__ __forceinline__ double fd_lx_reg(const double* w, double vx, double l
 // contracted path D_z of D_x and D_y from register windows (1.79).
 // W, H: the largest tile of the instance (18 x 17 or 34 x 9).  The row pitch
 // W + 16 puts consecutive pairs of a W-wide tile in consecutive banks across
-// a row's end.
-template <bool CONTRACT, int W, int H>
+// a row's end.  NC: components of a vertex in out; kDvCon stores the
+// derivatives of chi and g~ (grid y: these 7 variables) and no advection sums.
+template <bool CONTRACT, int W, int H, int NC = kDvComponents>
 __global__ void __launch_bounds__(kDvMaxThreads, 3)
 k_deriv(Grid g, DevParams P, const double* __restrict__ u, double* __restrict__ out, DerivTile T,
         int block0) {
@@ -158,6 +160,7 @@ k_deriv(Grid g, DevParams P, const double* __restrict__ u, double* __restrict__ 
   const int nn0 = g.nn[0], sk = nn0 * g.nn[1];
   const int n0 = g.nx[0] + 1, n1 = g.nx[1] + 1;
   constexpr int np = kDvGroup;  // stride of the components of a vertex
+  constexpr bool sums = NC == kDvComponents;
   const bool hess = f < kDvHess, grad = f < kDvHess + kDvGrad;
 
   const double* U = u + (int64_t)b * NVAR * g.nvol;
@@ -231,7 +234,7 @@ k_deriv(Grid g, DevParams P, const double* __restrict__ u, double* __restrict__ 
     w1[q] = col1 ? __ldg(z + 1) : 0.0;
   }
   const double* bp = U + (int64_t)Z4C_BETAX * g.nvol + gp;
-  double* const ob0 = out + blockIdx.z * dv_doubles((int64_t)T.nk * n1 * n0);
+  double* const ob0 = out + blockIdx.z * dv_doubles((int64_t)T.nk * n1 * n0, NC);
   int l = ((k0 - NG - T.ks) * n1 + j0 + ty - NG) * n0 + i0 + tx - NG;
   const int kd0 = grad ? (hess ? 9 * f : kDvFirst + 3 * (f - kDvHess)) : 0;
   auto advect = [&](const double* line, double v, int a) {
@@ -266,11 +269,13 @@ k_deriv(Grid g, DevParams P, const double* __restrict__ u, double* __restrict__ 
   for (int k = k0; k <= k1; ++k) {
     // the shift, its latency behind the barrier and the inner pass
     double be0[3], be1[3];
+    if constexpr (sums) {
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      const double* p = bp + a * g.nvol + (int64_t)k * sk;
-      be0[a] = act0 ? __ldg(p) : 0.0;
-      be1[a] = act1 ? __ldg(p + 1) : 0.0;
+      for (int a = 0; a < 3; ++a) {
+        const double* p = bp + a * g.nvol + (int64_t)k * sk;
+        be0[a] = act0 ? __ldg(p) : 0.0;
+        be1[a] = act1 ? __ldg(p + 1) : 0.0;
+      }
     }
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();
@@ -286,17 +291,15 @@ k_deriv(Grid g, DevParams P, const double* __restrict__ u, double* __restrict__ 
             fd7(w1[2], w1[3], w1[4], w1[6], w1[7], w1[8], cs[2]));
     if (act0) {
       // component q of the two vertices
-      double* const o0 =
-          ob0 + (int64_t)(l / kDvGroup) * (kDvComponents * kDvGroup) + l % kDvGroup;
+      double* const o0 = ob0 + (int64_t)(l / kDvGroup) * (NC * kDvGroup) + l % kDvGroup;
       const int l1 = l + 1;
-      double* const o1 =
-          ob0 + (int64_t)(l1 / kDvGroup) * (kDvComponents * kDvGroup) + l1 % kDvGroup;
+      double* const o1 = ob0 + (int64_t)(l1 / kDvGroup) * (NC * kDvGroup) + l1 % kDvGroup;
       auto put = [&](int q, double v0, double v1) {
         o0[q * np] = v0;
         if (act1) o1[q * np] = v1;
       };
       const double* c = fs + (unsigned)k % ring * plane + own;
-      double x[10], acc0, acc1;
+      double x[10], acc0 = 0., acc1 = 0.;
       row10(c, x);
       if (grad) {
         put(kd0, fd7(x[1], x[2], x[3], x[5], x[6], x[7], cs[0]),
@@ -305,8 +308,10 @@ k_deriv(Grid g, DevParams P, const double* __restrict__ u, double* __restrict__ 
           put(kd0 + 3, fd7xx(x[1], x[2], x[3], x[4], x[5], x[6], x[7], cs[3]),
               fd7xx(x[2], x[3], x[4], x[5], x[6], x[7], x[8], cs[3]));
       }
-      acc0 = 0. + advect(x, be0[0], 0);
-      acc1 = 0. + advect(x + 1, be1[0], 0);
+      if constexpr (sums) {
+        acc0 += advect(x, be0[0], 0);
+        acc1 += advect(x + 1, be1[0], 0);
+      }
       double y0[9], y1[9];
 #pragma unroll
       for (int q = 0; q < 9; ++q) {
@@ -314,11 +319,13 @@ k_deriv(Grid g, DevParams P, const double* __restrict__ u, double* __restrict__ 
         y0[q] = v.x;
         y1[q] = v.y;
       }
-      acc0 += advect(y0, be0[1], 1);
-      acc1 += advect(y1, be1[1], 1);
-      acc0 += advect(w0, be0[2], 2);
-      acc1 += advect(w1, be1[2], 2);
-      put(kDvAdv + n, acc0, acc1);
+      if constexpr (sums) {
+        acc0 += advect(y0, be0[1], 1);
+        acc1 += advect(y1, be1[1], 1);
+        acc0 += advect(w0, be0[2], 2);
+        acc1 += advect(w1, be1[2], 2);
+        put(kDvAdv + n, acc0, acc1);
+      }
       if (hess) {
         put(kd0 + 6, fd7xx(y0[1], y0[2], y0[3], y0[4], y0[5], y0[6], y0[7], cs[4]),
             fd7xx(y1[1], y1[2], y1[3], y1[4], y1[5], y1[6], y1[7], cs[4]));
@@ -403,7 +410,8 @@ inline DerivLaunch deriv_launch(const Grid& g, int nblk, int ks, int nk) {
   return L;
 }
 
-// for_deriv_chunks on the passes' scratch: launch(b, nb, ks, nk, scratch).
+// for_deriv_chunks on the right-hand side's scratch: launch(b, nb, ks, nk,
+// scratch).
 template <class Launch>
 inline void for_deriv_chunks(const Grid& g, int block0, int nblk, const RhsScratch& sc,
                              Launch launch) {

@@ -1005,22 +1005,21 @@ __global__ void k_adm_to_z4c_gam(Grid g, DevParams P, const double* __restrict__
 }
 
 // ADMConstraints on the interior vertices of the slab, one warp per 32, the
-// derivatives of chi and g~ from the derivative pass staged in shared memory
-// (the first 63 components); those of K_ab read through L1.  con is zero
+// derivatives of chi and g~ from the derivative pass staged in shared memory;
+// those of K_ab read through L1.  con is zero
 // elsewhere (the launcher clears it).  256 blocks of 16^3, ADM variables,
-// constraints and norms together: 0.96 ms, against 2.02 with the mixed
+// constraints and norms together: 0.91 ms, against 2.02 with the mixed
 // derivatives as 36-point stencils in place (1.79 of it).
-constexpr int kConComponents = 9 * 7;
 __global__ void __launch_bounds__(kDvGroup)
 k_adm_constraints(Grid g, DevParams P, const double* __restrict__ adm,
                   const double* __restrict__ u, const double* __restrict__ D,
                   double* __restrict__ con, const double* __restrict__ xf, int block0, int ks,
                   int nk) {
-  __shared__ __align__(16) double sm[kConComponents * kDvGroup];
+  __shared__ __align__(16) double sm[kDvCon * kDvGroup];
   const int n0 = g.nx[0] + 1, n1 = g.nx[1] + 1, np = nk * n1 * n0;
   const int l = (int)(blockIdx.x * kDvGroup + threadIdx.x);
-  stage_components<kConComponents>(
-      sm, D + blockIdx.y * dv_doubles(np) + (int64_t)blockIdx.x * (kDvComponents * kDvGroup));
+  stage_components<kDvCon>(
+      sm, D + blockIdx.y * dv_doubles(np, kDvCon) + (int64_t)blockIdx.x * (kDvCon * kDvGroup));
   asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
   __syncwarp();
   if (l >= np) return;
@@ -1312,6 +1311,8 @@ int allow_slab_smem() {
   };
   raise((const void*)k_deriv<false, 18, 17>, kDvMaxSmem);
   raise((const void*)k_deriv<false, 34, 9>, kDvMaxSmem);
+  raise((const void*)k_deriv<false, 18, 17, kDvCon>, kDvMaxSmem);
+  raise((const void*)k_deriv<false, 34, 9, kDvCon>, kDvMaxSmem);
   raise((const void*)k_point, kStageBytes);
   if (e == cudaSuccess) e = prefer_l1();
   if (e == cudaSuccess) e = (cudaError_t)allow_deriv_smem_fast();
@@ -1438,6 +1439,10 @@ void launch_stage_bt(const Grid& g, const DevParams& P, const double* u, const R
 }
 
 int64_t rhs_scratch_doubles(const Grid& g) { return dv_doubles(interior_count(g)); }
+int64_t con_scratch_share(const Grid& g) {
+  return dv_con_share(interior_count(g), (int64_t)(g.nx[0] + 1) * (g.nx[1] + 1), kDvCon,
+                      g.nblocks);
+}
 
 // Slot of every direction in the neighbour list (mesh_topology.cpp:329-960
 // order, the c_dirs table of the context), indexed (o0+1) + 3(o1+1) + 9(o2+1).
@@ -1573,19 +1578,22 @@ void launch_adm_to_z4c(const Grid& g, const DevParams& P, const double* adm, dou
       div_up(n, kPointThreads), kPointThreads, 0, st>>>(g, P, u, block0, nblk, 0);
 }
 
-int launch_adm_constraints(const Grid& g, const DevParams& P, const RhsScratch& sc,
+int launch_adm_constraints(const Grid& g, const DevParams& P, const ConScratch& sc,
                            const double* adm, const double* u, double* con, const double* xf,
                            int block0, int nblk, cudaStream_t st) {
   const cudaError_t e =
       cudaMemsetAsync(con + (int64_t)block0 * Z4C_NCON * g.nvol, 0,
                       sizeof(double) * (size_t)Z4C_NCON * g.nvol * nblk, st);
   if (e != cudaSuccess) return (int)e;
-  for_deriv_chunks(g, block0, nblk, sc, [&](int b, int nb, int ks, int nk, double* D) {
+  for_deriv_chunks(g.nx, block0, nblk, kDvCon, sc.share,
+                   [&](int b, int nb, int ks, int nk, int64_t at) {
+    double* const D = sc.base + at;
     DerivLaunch L = deriv_launch(g, nb, ks, nk);
-    L.grid.y = kConComponents / 9;
+    L.grid.y = kDvCon / 9;
     COUNTED
-    (L.narrow ? k_deriv<false, 18, 17> : k_deriv<false, 34, 9>)<<<L.grid, L.threads, L.smem,
-                                                                  st>>>(g, P, u, D, L.T, b);
+    (L.narrow ? k_deriv<false, 18, 17, kDvCon>
+              : k_deriv<false, 34, 9, kDvCon>)<<<L.grid, L.threads, L.smem, st>>>(g, P, u, D, L.T,
+                                                                                  b);
     const int64_t np = (int64_t)nk * (g.nx[1] + 1) * (g.nx[0] + 1);
     COUNTED
     k_adm_constraints<<<dim3(div_up(np, kDvGroup), nb), kDvGroup, 0, st>>>(

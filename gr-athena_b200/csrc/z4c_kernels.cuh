@@ -69,6 +69,13 @@ struct RhsScratch {
 constexpr int kSdComponents = 33;
 // Scratch doubles per block of the derivative pass.
 int64_t rhs_scratch_doubles(const Grid& g);
+// The constraints' derivatives have a scratch of their own, again a share per
+// block: a constraint evaluation may run beside a right-hand side.
+struct ConScratch {
+  double* base;
+  int64_t share;
+};
+int64_t con_scratch_share(const Grid& g);
 
 // Launch shape of the right-hand-side passes: threads per CTA of the
 // Kreiss-Oliger and stage pass (128, 256, 512) and the number of z-slabs per
@@ -158,8 +165,8 @@ void launch_z4c_to_adm(const Grid& g, const DevParams& P, const double* u, doubl
 // alg = 0 leaves out the final AlgConstr (the adjoint's recomputation)
 void launch_adm_to_z4c(const Grid& g, const DevParams& P, const double* adm, double* u,
                        double* guu_scratch, int block0, int nblk, cudaStream_t st, int alg = 1);
-// Uses the right-hand-side scratch; returns a cudaError_t value.
-int launch_adm_constraints(const Grid& g, const DevParams& P, const RhsScratch& sc,
+// Returns a cudaError_t value.
+int launch_adm_constraints(const Grid& g, const DevParams& P, const ConScratch& sc,
                            const double* adm, const double* u, double* con, const double* xf,
                            int block0, int nblk, cudaStream_t st);
 // Z4cWeyl on blocks [block0, block0+nblk): the stored first derivatives of u

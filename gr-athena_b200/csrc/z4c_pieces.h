@@ -37,6 +37,15 @@ inline int64_t dv_context_share(int64_t parts, int64_t whole, int nblocks) {
   const bool all = whole <= parts + parts / 16 || whole * nblocks <= (int64_t)1 << 29;
   return all && whole > parts ? whole : parts;
 }
+// A block's share of the constraints' own scratch, nc components of npts
+// vertices in planes of `plane`: whole, but no more than 1 GiB on the mesh while
+// a share still holds a plane (512 blocks of 16^3 run as two groups then, at
+// the same time as at once).
+inline int64_t dv_con_share(int64_t npts, int64_t plane, int nc, int nblocks) {
+  const int64_t whole = dv_doubles(npts, nc), least = dv_doubles(plane + kDvGroup, nc);
+  const int64_t cap = dv_share((int64_t)1 << 27, nblocks);
+  return whole <= cap ? whole : least <= cap ? cap : least;
+}
 
 // Runs the derivative and pointwise passes on blocks block0 .. block0 + nblk - 1
 // of nx cells in pieces whose scratch fits these blocks' shares: all at once,

@@ -168,7 +168,11 @@ int z4c_create_refined(const z4c_mesh_desc_t *mesh, int nblocks, const long long
 int z4c_refined_neighbours(const z4c_mesh_desc_t *mesh, int nblocks, const long long *locs,
                            int block, int *out);
 int z4c_destroy(z4c_ctx *ctx);
-/* Work is enqueued on this CUDA stream (a cudaStream_t; NULL = default). */
+/* Work is enqueued on this CUDA stream (a cudaStream_t; NULL = default).
+ * Nothing orders the new stream behind the old one.  Calls enqueued on
+ * different streams may overlap where the registers they use do not and they
+ * either work on different MeshBlocks or are right-hand sides (or psi4) beside
+ * constraints; order all others, e.g. by an event. */
 int z4c_set_stream(z4c_ctx *ctx, void *stream);
 int z4c_sync(z4c_ctx *ctx);
 /* Geometry queries: blocks, vertices per block axis, variables of a register,

@@ -26,3 +26,7 @@ extern "C" int pc_chunks(const int nx[3], int block0, int nblk, int components, 
 extern "C" long long pc_context_share(long long parts, long long whole, int nblocks) {
   return z4c::dv_context_share(parts, whole, nblocks);
 }
+
+extern "C" long long pc_con_share(long long npts, long long plane, int nc, int nblocks) {
+  return z4c::dv_con_share(npts, plane, nc, nblocks);
+}

@@ -50,3 +50,33 @@ def test_blocks_on_alternating_streams(nx, contract):
     ctx.close()
     for a, b in zip(alone, both):
         assert np.array_equal(a, b, equal_nan=True)  # psi4 is NaN outside the interior
+
+
+@pytest.mark.parametrize("contract", [False, True])
+@pytest.mark.parametrize("nx", [(16, 16, 16), (40, 24, 22)])
+def test_constraints_beside_right_hand_sides(nx, contract):
+    """Constraints of single blocks and of the mesh on one stream, right-hand
+    sides of the mesh on another: the bits of the same calls on one stream."""
+    import torch
+    Z, ctx = make((3, 1, 1), nx, contract)
+    ctx.Z4cToADM()
+
+    def run(streams):
+        for reg in (Z.REG_RHS, Z.REG_CON):
+            ctx.upload(reg, np.zeros(ctx.shape(reg)))
+        torch.cuda.synchronize()
+        for _ in range(12):
+            ctx.set_stream(streams[0].cuda_stream)
+            ctx.Z4cRHS()
+            ctx.set_stream(streams[-1].cuda_stream)
+            for b in (0, 1, 2, -1):
+                ctx.ADMConstraints(block=b)
+        torch.cuda.synchronize()
+        return ctx.download(Z.REG_RHS), ctx.download(Z.REG_CON)
+
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    alone = run(streams[:1])
+    both = run(streams)
+    ctx.close()
+    for a, b in zip(alone, both):
+        assert np.array_equal(a, b)

@@ -15,6 +15,7 @@ from z4c_testlib import ROOT
 
 SRC = os.path.join(ROOT, "tests", "pieces", "pieces_check.cpp")
 COMPONENTS = 136  # of the right-hand side, per interior vertex
+CON = 63  # of the constraints
 LL = C.c_longlong
 
 
@@ -23,7 +24,7 @@ def pc(tmp_path_factory):
     out = str(tmp_path_factory.mktemp("pc") / "pc.so")
     subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-o", out, SRC], check=True)
     L = C.CDLL(out)
-    for f in (L.pc_doubles, L.pc_share, L.pc_context_share):
+    for f in (L.pc_doubles, L.pc_share, L.pc_context_share, L.pc_con_share):
         f.restype = LL
     return L
 
@@ -100,3 +101,17 @@ def test_context_shares(pc):
             assert share <= max(parts(nx) + parts(nx) // 16, 2 ** 29 // nblocks) + 32
             check(pc, nx, nblocks - 1, 1, COMPONENTS, share)
             check(pc, nx, 0, min(nblocks, 3), COMPONENTS, share)
+
+
+def test_constraint_shares(pc):
+    """The constraints' scratch: whole blocks up to 1 GiB on the mesh, at least
+    a plane of every block."""
+    for nx in [(8, 8, 8), (200, 200, 8), (16, 16, 16), (24, 24, 24), (33, 8, 12), (160, 160, 160)]:
+        plane, nk = (nx[0] + 1) * (nx[1] + 1), nx[2] + 1
+        per = pc.pc_doubles(LL(plane * nk), CON)
+        for nblocks in (1, 3, 128, 512, 3424, 20000):
+            share = pc.pc_con_share(LL(plane * nk), LL(plane), CON, nblocks)
+            assert share % 32 == 0 and share <= per
+            assert share == per or share * nblocks <= 2 ** 27 or share <= CON * (plane + 64)
+            check(pc, nx, nblocks - 1, 1, CON, share)
+            check(pc, nx, 0, min(nblocks, 5), CON, share)
