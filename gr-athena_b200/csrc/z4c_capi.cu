@@ -320,7 +320,7 @@ void free_ctx(z4c_ctx* c) {
   c->reg[Z4C_REG_TAN] = c->reg[Z4C_REG_ADJ] = c->reg[Z4C_REG_ADM_ADJ] = nullptr;
   for (auto& r : c->reg)
     if (r) cudaFree(r);
-  for (void* p : {(void*)c->un, (void*)c->guu, (void*)c->sd, (void*)c->con.base, (void*)c->xf, (void*)c->xv, (void*)c->dxd, (void*)c->fd,
+  for (void* p : {(void*)c->un, (void*)c->guu, (void*)c->sd, (void*)c->xf, (void*)c->xv, (void*)c->dxd, (void*)c->fd,
                   (void*)c->nbr, (void*)c->partials, (void*)c->flag, (void*)c->trk})
     if (p) cudaFree(p);
   for (auto& w : c->waves) wave_free(&w);
@@ -385,7 +385,8 @@ namespace {
 // A context on a uniform block grid (locs == nullptr) or on the nblocks
 // blocks of a refined mesh given by their logical locations in gid order.
 int create_impl(const z4c_mesh_desc_t* mesh, const z4c_params_t* params, int integrator,
-                int nblocks_ml, const long long* locs, z4c_ctx** out) {
+                int nblocks_ml, const long long* locs, z4c_ctx** out,
+                bool merged = false) {
   if (!mesh || !params || !out) return fail(Z4C_EINVAL, "null argument");
   *out = nullptr;
   if (integrator != Z4C_INTEG_RK4 && integrator != Z4C_INTEG_BT_RK4)
@@ -555,18 +556,26 @@ int create_impl(const z4c_mesh_desc_t* mesh, const z4c_params_t* params, int int
   if (rc == Z4C_OK && integrator == Z4C_INTEG_BT_RK4) rc = alloc((void**)&c->un, b22);
   if (rc == Z4C_OK) rc = alloc((void**)&c->guu, sizeof(double) * 6 * (size_t)g.nvol * nb);
   {
-    const int64_t npts = interior_count(g);
-    c->scratch_share = dv_context_share((int64_t)kSdComponents * g.nvol + 28 * npts,
-                                        rhs_scratch_doubles(g), nb);
-    if (rc == Z4C_OK)
-      rc = alloc((void**)&c->sd, sizeof(double) * (size_t)c->scratch_share * nb);
+    DvShares best, least, got;
+    scratch_shares(g, &best, &least);
+    if (merged) {
+      // the constraints are evaluated on the blocks; the fixed instance's
+      // stencils read the stored first derivatives only
+      best.con = least.con = 0;
+      if (has_merged_geometry(g)) best.rhs = least.rhs;
+    }
+    if (rc == Z4C_OK &&
+        !dv_reserve(best, least, nb, [&](int64_t n) {
+          rc = alloc((void**)&c->sd, sizeof(double) * (size_t)n);
+          return rc == Z4C_OK;
+        }, &got))
+      c->sd = nullptr;
     if (rc == Z4C_OK) {
+      c->scratch_share = got.rhs;
+      c->con = ConScratch{c->sd + got.rhs * nb, got.con};
       c->rsum = c->scratch().rsum;
       c->lv = c->scratch().lv;
     }
-    c->con.share = con_scratch_share(g);
-    if (rc == Z4C_OK)
-      rc = alloc((void**)&c->con.base, sizeof(double) * (size_t)c->con.share * nb);
   }
   if (rc == Z4C_OK) rc = alloc((void**)&c->xf, sizeof(double) * c->h_xf.size());
   if (rc == Z4C_OK) rc = alloc((void**)&c->xv, sizeof(double) * c->h_xv.size());
@@ -1390,7 +1399,7 @@ int merged_evolve(z4c_ctx* c, double dt, int nsteps, int with_constraints) {
       d.nb[a] = 1;
     }
     z4c_ctx* m = nullptr;
-    int rc = create_impl(&d, &c->params, c->integrator, 0, nullptr, &m);
+    int rc = create_impl(&d, &c->params, c->integrator, 0, nullptr, &m, true);
     if (rc) return rc;
     m->merge = false;
     // a periodic single block still runs the exchange (with itself)

@@ -67,7 +67,7 @@ struct z4c_ctx {
   double* rsum = nullptr; // per vertex, then Ricci sums, 6 values per interior
   double* lv = nullptr;   // vertex, then 22 values per interior vertex
   int64_t scratch_share = 0;  // doubles of each block's share at sd
-  ConScratch con{};           // the constraints' scratch
+  ConScratch con{};           // the constraints' scratch, behind sd's shares
   double* xf = nullptr;   // [nblocks][nn0+nn1+nn2]
   double* xv = nullptr;   // [nblocks][nn0+nn1+nn2-3]
   double* dxd = nullptr;  // [nblocks][3] vertex spacing

@@ -1438,10 +1438,11 @@ void launch_stage_bt(const Grid& g, const DevParams& P, const double* u, const R
   }
 }
 
-int64_t rhs_scratch_doubles(const Grid& g) { return dv_doubles(interior_count(g)); }
-int64_t con_scratch_share(const Grid& g) {
-  return dv_con_share(interior_count(g), (int64_t)(g.nx[0] + 1) * (g.nx[1] + 1), kDvCon,
-                      g.nblocks);
+void scratch_shares(const Grid& g, DvShares* best, DvShares* least) {
+  const int64_t npts = interior_count(g);
+  *least = dv_least_shares(kSdComponents * g.nvol + 28 * npts,
+                           (int64_t)(g.nx[0] + 1) * (g.nx[1] + 1), kDvCon);
+  *best = dv_best_shares(*least, dv_doubles(npts), npts, kDvCon, g.nblocks);
 }
 
 // Slot of every direction in the neighbour list (mesh_topology.cpp:329-960

@@ -4,6 +4,7 @@
 #pragma once
 
 #include "z4c_common.cuh"
+#include "z4c_pieces.h"
 
 namespace z4c {
 
@@ -67,15 +68,14 @@ struct RhsScratch {
   int64_t share;
 };
 constexpr int kSdComponents = 33;
-// Scratch doubles per block of the derivative pass.
-int64_t rhs_scratch_doubles(const Grid& g);
 // The constraints' derivatives have a scratch of their own, again a share per
 // block: a constraint evaluation may run beside a right-hand side.
 struct ConScratch {
   double* base;
   int64_t share;
 };
-int64_t con_scratch_share(const Grid& g);
+// The shares of a block that a context should have, and the least it runs with.
+void scratch_shares(const Grid& g, DvShares* best, DvShares* least);
 
 // Launch shape of the right-hand-side passes: threads per CTA of the
 // Kreiss-Oliger and stage pass (128, 256, 512) and the number of z-slabs per

@@ -3,6 +3,7 @@
 #pragma once
 
 #include <cstdint>
+#include <initializer_list>
 
 #ifdef __CUDACC__
 #define Z4C_PIECES_HD __host__ __device__ __forceinline__
@@ -28,23 +29,43 @@ Z4C_PIECES_HD constexpr int64_t dv_doubles(int64_t vertices, int components) {
 inline int64_t dv_share(int64_t cap, int nblocks) {
   return cap / nblocks / kDvGroup * kDvGroup;
 }
-// A context's share of a block: what the diagnostics and the adjoint need
-// (parts), or every component of the derivative pass (whole) where that is at
-// most a little more, or small on the mesh (512 Mi doubles); otherwise the
-// passes run in pieces that fit.
-inline int64_t dv_context_share(int64_t parts, int64_t whole, int nblocks) {
-  parts = (parts + kDvGroup - 1) / kDvGroup * kDvGroup;
-  const bool all = whole <= parts + parts / 16 || whole * nblocks <= (int64_t)1 << 29;
-  return all && whole > parts ? whole : parts;
+// A block's shares of a context's scratch.
+struct DvShares {
+  int64_t rhs;  // right-hand side, diagnostics and adjoint
+  int64_t con;  // constraints
+};
+// The least a context runs with: what the diagnostics and the adjoint need
+// (parts), and a plane of the constraints' nc components.
+inline DvShares dv_least_shares(int64_t parts, int64_t plane, int nc) {
+  return {(parts + kDvGroup - 1) / kDvGroup * kDvGroup, dv_doubles(plane + kDvGroup, nc)};
 }
-// A block's share of the constraints' own scratch, nc components of npts
-// vertices in planes of `plane`: whole, but no more than 1 GiB on the mesh while
-// a share still holds a plane (512 blocks of 16^3 run as two groups then, at
-// the same time as at once).
-inline int64_t dv_con_share(int64_t npts, int64_t plane, int nc, int nblocks) {
-  const int64_t whole = dv_doubles(npts, nc), least = dv_doubles(plane + kDvGroup, nc);
-  const int64_t cap = dv_share((int64_t)1 << 27, nblocks);
-  return whole <= cap ? whole : least <= cap ? cap : least;
+// What serves the passes best: every component of the right-hand side (whole)
+// where that is at most a little more, or small on the mesh (512 Mi doubles);
+// every one of the constraints', but no more than 1 GiB on the mesh (512 blocks
+// of 16^3 run as two groups then, at the same time as at once).  The passes
+// run in pieces that fit.
+inline DvShares dv_best_shares(const DvShares& least, int64_t whole, int64_t npts, int nc,
+                               int nblocks) {
+  DvShares s = least;
+  if (whole > s.rhs &&
+      (whole <= s.rhs + s.rhs / 16 || whole * nblocks <= (int64_t)1 << 29))
+    s.rhs = whole;
+  const int64_t con = dv_doubles(npts, nc), cap = dv_share((int64_t)1 << 27, nblocks);
+  if (con <= cap) s.con = con;
+  else if (cap > s.con) s.con = cap;
+  return s;
+}
+// Allocates the scratch of nblocks blocks: the best shares, or, where the
+// device does not hold those, the least.  alloc(doubles) says whether it could;
+// returns whether one of them did, its shares in *got.
+template <class Alloc>
+inline bool dv_reserve(const DvShares& best, const DvShares& least, int nblocks, Alloc alloc,
+                       DvShares* got) {
+  for (const DvShares* s : {&best, &least}) {
+    *got = *s;
+    if (alloc((s->rhs + s->con) * nblocks)) return true;
+  }
+  return false;
 }
 
 // Runs the derivative and pointwise passes on blocks block0 .. block0 + nblk - 1

@@ -24,7 +24,7 @@ def pc(tmp_path_factory):
     out = str(tmp_path_factory.mktemp("pc") / "pc.so")
     subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-o", out, SRC], check=True)
     L = C.CDLL(out)
-    for f in (L.pc_doubles, L.pc_share, L.pc_context_share, L.pc_con_share):
+    for f in (L.pc_doubles, L.pc_share):
         f.restype = LL
     return L
 
@@ -72,46 +72,59 @@ def test_pieces_stay_inside_the_shares_and_cover_the_mesh(pc, nx):
                 check(pc, nx, b, total - b, COMPONENTS, share)
 
 
-def parts(nx):  # 33 values per vertex and 28 per interior vertex
+def shares(pc, nx, nblocks):
+    """(rhs, con) of the least and of the best shares of a context's scratch."""
     nn = [n + 9 for n in nx]
-    return 33 * nn[0] * nn[1] * nn[2] + 28 * (nx[0] + 1) * (nx[1] + 1) * (nx[2] + 1)
+    plane, npts = (nx[0] + 1) * (nx[1] + 1), (nx[0] + 1) * (nx[1] + 1) * (nx[2] + 1)
+    # the diagnostics and the adjoint: 33 values per vertex, 28 per interior one
+    parts = 33 * nn[0] * nn[1] * nn[2] + 28 * npts
+    least, best = (LL * 2)(), (LL * 2)()
+    pc.pc_shares(LL(parts), LL(pc.pc_doubles(LL(npts), COMPONENTS)), LL(npts), LL(plane), CON,
+                 nblocks, least, best)
+    return parts, tuple(least), tuple(best)
 
 
 def test_groups_of_an_odd_number_of_blocks(pc):
     """Three blocks of 112^3 whose scratch holds 1.5 of them: one block at a
     time."""
     nx = (112, 112, 112)
-    per = pc.pc_doubles(LL(113 ** 3), COMPONENTS)
-    share = pc.pc_context_share(LL(parts(nx)), LL(per), 3)
-    assert share < per
+    _, _, (share, _) = shares(pc, nx, 3)
+    assert share < pc.pc_doubles(LL(113 ** 3), COMPONENTS)
     rows = check(pc, nx, 0, 3, COMPONENTS, share)
     assert [r[:4] for r in rows] == [(b, 1, 0, 113) for b in range(3)]
 
 
-def test_context_shares(pc):
-    """A context's share holds the three arrays of the diagnostics and the
-    adjoint, and planes enough for the derivative pass on one block."""
-    for nx in [(8, 8, 8), (8, 8, 200), (200, 200, 8), (16, 16, 16), (24, 24, 24), (33, 8, 12),
-               (48, 48, 48), (160, 160, 160), (300, 300, 300)]:
-        plane, nk = (nx[0] + 1) * (nx[1] + 1), nx[2] + 1
-        per = pc.pc_doubles(LL(plane * nk), COMPONENTS)
-        for nblocks in (1, 3, 128, 3424):
-            share = pc.pc_context_share(LL(parts(nx)), LL(per), nblocks)
-            assert share >= parts(nx) and share % 32 == 0
-            assert share <= max(parts(nx) + parts(nx) // 16, 2 ** 29 // nblocks) + 32
-            check(pc, nx, nblocks - 1, 1, COMPONENTS, share)
-            check(pc, nx, 0, min(nblocks, 3), COMPONENTS, share)
+@pytest.mark.parametrize("nx", [(8, 8, 8), (8, 8, 200), (200, 200, 8), (16, 16, 16),
+                                (24, 24, 24), (33, 8, 12), (48, 48, 48), (160, 160, 160),
+                                (300, 300, 300)])
+def test_context_shares(pc, nx):
+    """A context's shares hold the three arrays of the diagnostics and the
+    adjoint, and planes enough for both passes on one block; the best ones are
+    bounded."""
+    for nblocks in (1, 3, 128, 512, 3424, 20000):
+        parts, least, best = shares(pc, nx, nblocks)
+        assert parts <= least[0] <= parts + 31
+        assert least[0] <= best[0] and least[1] <= best[1]
+        assert best[0] <= max(least[0] + least[0] // 16, 2 ** 29 // nblocks)
+        assert best[1] <= max(least[1], 2 ** 27 // nblocks)
+        for s in (least, best):
+            assert s[0] % 32 == 0 and s[1] % 32 == 0
+            for comps, share in ((COMPONENTS, s[0]), (CON, s[1])):
+                check(pc, nx, nblocks - 1, 1, comps, share)
+                check(pc, nx, 0, min(nblocks, 5), comps, share)
 
 
-def test_constraint_shares(pc):
-    """The constraints' scratch: whole blocks up to 1 GiB on the mesh, at least
-    a plane of every block."""
-    for nx in [(8, 8, 8), (200, 200, 8), (16, 16, 16), (24, 24, 24), (33, 8, 12), (160, 160, 160)]:
-        plane, nk = (nx[0] + 1) * (nx[1] + 1), nx[2] + 1
-        per = pc.pc_doubles(LL(plane * nk), CON)
-        for nblocks in (1, 3, 128, 512, 3424, 20000):
-            share = pc.pc_con_share(LL(plane * nk), LL(plane), CON, nblocks)
-            assert share % 32 == 0 and share <= per
-            assert share == per or share * nblocks <= 2 ** 27 or share <= CON * (plane + 64)
-            check(pc, nx, nblocks - 1, 1, CON, share)
-            check(pc, nx, 0, min(nblocks, 5), CON, share)
+def test_scratch_falls_back_when_the_device_is_full(pc):
+    """A device that does not hold the best scratch gets the least one; one that
+    does not hold that either refuses."""
+    for nx, nblocks in (((128, 128, 128), 1), ((32, 32, 32), 64), ((16, 16, 16), 512)):
+        _, least, best = shares(pc, nx, nblocks)
+        for room, expect in ((sum(best) * nblocks, best), (sum(best) * nblocks - 1, least),
+                             (sum(least) * nblocks, least), (sum(least) * nblocks - 1, None)):
+            got, n = (LL * 2)(), LL()
+            ok = pc.pc_reserve((LL * 2)(*least), (LL * 2)(*best), nblocks, LL(room), got,
+                               C.byref(n))
+            assert bool(ok) == (expect is not None)
+            assert n.value == (sum(expect) * nblocks if expect else 0)
+            if expect:
+                assert tuple(got) == expect
