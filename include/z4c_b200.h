@@ -392,8 +392,8 @@ int z4c_get_tile(const z4c_ctx *ctx, int tile_out[3]);
  * Its right-hand side agrees with the exact path's (which matches the
  * reference bit for bit) to round-off, within the 1e-12 relative bound per
  * evaluation; meshes with gr_sommerfeld faces and the Butcher integrator keep
- * the exact path.  Off by default; switching drops the captured step graph,
- * and the autotuner times the path that is switched on. */
+ * the exact path.  Off by default; switching drops the captured step graph.
+ * The launch shape (z4c_set_tile) is the exact path's. */
 int z4c_set_contract(z4c_ctx *ctx, int on);
 /* Register budget of the per-vertex right-hand-side pass (no reference
  * counterpart), 0 or 168: kept for callers and reported back; the pass has one
@@ -420,11 +420,13 @@ int z4c_get_contract(const z4c_ctx *ctx, int *on);
 int z4c_set_merged(z4c_ctx *ctx, int on);
 int z4c_get_merged(const z4c_ctx *ctx, int *on);
 /* Autotuner (no reference counterpart): times one fused low-storage stage on
- * the context's current state for each candidate shape (the Ricci/main CTA
- * size first, then the column-pass shape; reps timed launches each after a
- * warm-up), keeps the fastest and drops the captured step graph.  Writes the
- * work register, u1 and rhs (u is untouched); call it between steps.
- * *best_ms (may be NULL) receives the stage time of the chosen shape. */
+ * the context's current state for each CTA size and slab count of the
+ * Kreiss-Oliger and stage pass (reps timed launches each after a warm-up),
+ * keeps the fastest and drops the captured step graph.  On the contracted
+ * path, whose launches follow from the mesh alone, it times the stage and
+ * leaves the shape.  Writes the work register, u1 and rhs (u is untouched);
+ * call it between steps.  *best_ms (may be NULL) receives the stage time of
+ * the chosen shape. */
 int z4c_autotune(z4c_ctx *ctx, int reps, float *best_ms);
 /* PunctureTracker (z4c/puncture_tracker.cpp): adds a tracker at pos; every
  * following step interpolates the shift at the tracker from the state at the

@@ -143,3 +143,15 @@ def test_launch_shapes_and_autotuner_leave_results_unchanged():
     with pytest.raises(Z.Z4cError):
         ctx.set_tile(100, 256, 2)
     ctx.close()
+
+
+def test_autotuner_leaves_the_shape_on_the_contracted_path():
+    """The contracted stage does not depend on the launch shape: the autotuner
+    reports its time and leaves the exact path's shape as it was."""
+    Z, ctx = mesh_ctx("outflow", nb=(2, 2, 2))
+    puncture_state(Z, ctx)
+    ctx.set_tile(64, 256, 2)
+    ctx.set_contract(True)
+    shape, ms = ctx.autotune(reps=2)
+    assert shape == (64, 256, 2) and ctx.get_tile() == (64, 256, 2) and ms > 0
+    ctx.close()
