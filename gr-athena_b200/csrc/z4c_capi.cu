@@ -1110,8 +1110,11 @@ int z4c_set_tile(z4c_ctx* ctx, int ti, int tj, int tk) {
   if (!valid_shape(sh))
     return fail(Z4C_EINVAL, "unsupported launch shape (%d, %d, %d): point threads 64/128/256, "
                 "column threads 128/256/512, column slabs 0-4", ti, tj, tk);
+  // the point threads select nothing, and the captured step stays
+  const bool same = sh.column_threads == ctx->shape.column_threads &&
+                    sh.column_slabs == ctx->shape.column_slabs;
   ctx->shape = sh;
-  drop_graph(ctx);
+  if (!same) drop_graph(ctx);
   return Z4C_OK;
 }
 
@@ -1119,10 +1122,7 @@ int z4c_set_point_regs(z4c_ctx* ctx, int regs) {
   if (!ctx) return fail(Z4C_EINVAL, "null context");
   if (regs != 0 && regs != kPointRegsHigh)
     return fail(Z4C_EINVAL, "register budget %d: 0 or %d", regs, kPointRegsHigh);
-  if (ctx->shape.point_regs != regs) {
-    ctx->shape.point_regs = regs;
-    drop_graph(ctx);
-  }
+  ctx->shape.point_regs = regs;
   return Z4C_OK;
 }
 
@@ -1412,13 +1412,7 @@ int merged_evolve(z4c_ctx* c, double dt, int nsteps, int with_constraints) {
   }
   z4c_ctx* m = c->merged;
   if (m->stream != c->stream) z4c_set_stream(m, c->stream);
-  if (m->shape.point_threads != c->shape.point_threads ||
-      m->shape.column_threads != c->shape.column_threads ||
-      m->shape.column_slabs != c->shape.column_slabs || m->shape.contract != c->shape.contract ||
-      m->shape.point_regs != c->shape.point_regs) {
-    m->shape = c->shape;
-    drop_graph(m);
-  }
+  m->shape = c->shape;  // contracted: its captured step reads nothing else of it
   if (m->ntrk != c->ntrk) {
     m->ntrk = c->ntrk;
     drop_graph(m);
