@@ -1,6 +1,6 @@
-"""The contracted path (z4c_set_contract: fused multiply-adds; advection,
-Kreiss-Oliger and the stage update in one per-variable column pass after the
-main pass) against the reference's own outputs.  Its right-hand side is not the
+"""The contracted path (z4c_set_contract: fused multiply-adds; the advection
+and Kreiss-Oliger sums formed with the derivatives, the stage update at the end
+of the pointwise pass) against the reference's own outputs.  Its right-hand side is not the
 reference's bit for bit, so every check is a bound:
 
   right-hand side      normwise relative 1e-12 per register (the FP64
@@ -140,9 +140,9 @@ def test_contract_switch_keeps_exact_path_exact():
 @pytest.mark.parametrize("contract", [False, True])
 @pytest.mark.parametrize("threads", [64, 128])
 def test_register_budget_changes_no_bits(contract, threads):
-    """The 168-register instances of the heavy passes compute the same
-    values as the 255-register ones (register allocation only), on 16^3
-    MeshBlocks where they apply."""
+    """The register budget and the point threads are kept for callers: both are
+    accepted and reported back, select nothing, and leave the captured step
+    in place."""
     import z4c_b200 as Z
     from z4c_b200 import initial_data as ID
     mesh = Z.Mesh((2, 2, 2), (16, 16, 16), (-4.0,) * 3, (4.0,) * 3, "outflow")
@@ -157,10 +157,16 @@ def test_register_budget_changes_no_bits(contract, threads):
         ctx.set_tile(threads, 128, 0)
         ctx.set_point_regs(regs)
         assert ctx.get_point_regs() == regs
+        assert ctx.get_tile() == (threads, 128, 0)
         ctx.Z4cRHS(Z.REG_U, Z.REG_RHS)
-        out.append(ctx.download(Z.REG_RHS))
+        rhs = ctx.download(Z.REG_RHS)
+        u = ctx.download(Z.REG_U)
+        ctx.evolve(0.05, 1)
+        out.append((rhs, ctx.download(Z.REG_U)))
+        ctx.upload(Z.REG_U, u)
     ctx.close()
-    assert np.array_equal(out[0], out[1])
+    assert np.array_equal(out[0][0], out[1][0])
+    assert np.array_equal(out[0][1], out[1][1])
 
 
 @pytest.mark.parametrize("nb,lim,steps", [
