@@ -121,19 +121,6 @@ __device__ __forceinline__ double fd_dxx(const double* __restrict__ u, int64_t s
   return out * cidx2;
 }
 
-// Mixed second derivative as the reference forms it: Dx along a of the
-// (rounded) Dx along b, evaluated at the six neighbours along a
-// (calculate_z4c_rhs.cpp:132,153,174-175).
-__device__ __forceinline__ double fd_dxy(const double* __restrict__ u, int64_t sa,
-                                         int64_t sb, double cidx1a, double cidx1b) {
-  double out = 0.;
-  out += -1. * (fd_dx(u - 3 * sa, sb, cidx1b) - fd_dx(u + 3 * sa, sb, cidx1b));
-  out += 9. * (fd_dx(u - 2 * sa, sb, cidx1b) - fd_dx(u + 2 * sa, sb, cidx1b));
-  out += -45. * (fd_dx(u - sa, sb, cidx1b) - fd_dx(u + sa, sb, cidx1b));
-  FD_FENCE();
-  return out * cidx1a;
-}
-
 // ---- linear algebra -------------------------------------------------------
 
 // index of the symmetric pair (a,b) in xx,xy,xz,yy,yz,zz order

@@ -124,8 +124,8 @@ __device__ __forceinline__ double fd_lx_reg(const double* w, double vx, double l
 // column per thread: 455 instructions per vertex and variable against 307).
 // The cost does not depend on the block's size, as the strides of the tile
 // are constants whatever those of the array.
-// Bound by shared-memory reads and issue at 15 warps per SM: 512 blocks of
-// 16^3, 1.17 ms, 4.06 GB of DRAM traffic (3.5 TB/s).  Together with the
+// Bound by shared-memory reads (its data pipe at 73% of its peak) at 14 warps
+// per SM: 512 blocks of 16^3, 1.19 ms, 4.05 GB of DRAM traffic (3.4 TB/s).  Together with the
 // pointwise pass (0.78 ms, 5.2 TB/s) it replaces stored first derivatives
 // (0.50 ms), Ricci (0.64), advection (0.59) and main (0.72) passes whose
 // stencils went to L1 and L2 at eight warps per SM.  Measured and slower: a

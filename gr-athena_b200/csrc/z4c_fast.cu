@@ -25,7 +25,7 @@ namespace {
 inline int div_up(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
 
 // One warp per 32 interior vertices, their operands staged in shared memory
-// (stage_group).  512 blocks of 16^3 with the stage update: 0.89 ms, 4.6 GB.
+// (stage_group).  512 blocks of 16^3 with the stage update: 0.89 ms, 5.2 GB.
 template <bool STAGE>
 __global__ void __launch_bounds__(kDvGroup)
 k_point_fast(Grid g, DevParams P, const double* __restrict__ u, const double* __restrict__ D,
@@ -70,12 +70,15 @@ k_point_fast(Grid g, DevParams P, const double* __restrict__ u, const double* __
 // One block whose strides are compile-time constants: the whole right-hand
 // side of a vertex from stencils in place (k_stencil_point, on the stored
 // first derivatives of k_prep; no spills at 254 registers), then one column
-// pass with the advection and Kreiss-Oliger sums and the stage update.  On
-// this grid faster than the derivative pass, whose scratch is 2.3 GB: a stage
-// takes 1.55 ms against 1.85 (1.81 with the Ricci sums in a pass of their own
-// and a branch on the shift's sign around the column pass's loads).  With
-// strides from the Grid it spills, and the derivative pass is the faster one
-// (64^3: 0.26 ms against 0.44).
+// pass with the advection and Kreiss-Oliger sums and the stage update.  A
+// stage takes 1.55 ms against 1.86 with the derivative pass (1.81 with the
+// Ricci sums in a pass of their own and a branch on the shift's sign around the
+// column pass's loads).  With strides from the Grid it spills (316 B), and the
+// derivative pass is the faster one (64^3: 0.26 ms against 0.44).  Instances of
+// other sizes, measured against the derivative pass, us a stage: 64^3 261 and
+// 260, 96^3 705 and 774, 112^3 1068 and 1323, 144^3 2216 and 2860, 160^3 3017
+// and 3548, 192^3 5900 and 6270.  So the instance pays for cubes from 96^3 on;
+// only the size that Z4C_MERGED_NX names (128 by default) is built.
 template <int THREADS, int NX>
 __global__ void __launch_bounds__(THREADS)
 k_stencil_point(Grid gin, DevParams P, const double* __restrict__ u,

@@ -8,17 +8,20 @@
 // device-wide synchronisation that cudaMalloc/cudaFree bring.  z4c_rhs needs a
 // context, and a context allocates its registers and scratch.  This entry
 // point takes the state and the output as plain device pointers and keeps the
-// scratch of the right-hand-side passes (the stored first derivatives, the
-// Ricci sums and the advection sums) in a fixed array compiled into the
-// library.
+// scratch of the right-hand-side passes (every derivative and advection sum of
+// an interior vertex) in a fixed array compiled into the library.
 //
 // The array: kScratchBytes = 64 MiB, a file-scope __device__ array.  Every GPU
 // that loads the library holds it until the process exits.  All calls share
 // it and it keeps the last call's contents: nothing in it has to start at
 // zero (each pass writes every entry it later reads), and two calls whose
 // work overlaps on the GPU (different streams, or different host threads)
-// race on it.  Blocks are processed in chunks that fit the array; a single
-// MeshBlock whose scratch does not fit is rejected.
+// race on it.  Blocks are processed in chunks, which the passes cut further
+// where their 136 components per interior vertex do not fit at once: into
+// groups of blocks, or slabs of one block's planes.  What one block may be and
+// how many make a chunk follows from 33 doubles per vertex and 28 per interior
+// vertex, the scratch of a context's share (z4c_pieces.h): the limit is part of
+// the interface, although the slabs would take larger blocks.
 //
 // The first call on a device: with CUDA's lazy module loading the address
 // lookup below is when the driver loads this library's device code on that
@@ -121,8 +124,7 @@ extern "C" int z4c_rhs_noalloc(const double* u, double* rhs, int nblocks, const 
   g.s[2] = (int64_t)g.nn[0] * g.nn[1];
   g.nvol = (int64_t)g.nn[0] * g.nn[1] * g.nn[2];
   const int64_t npts = interior_count(g);
-  // scratch per block: 33 stored first derivatives per vertex, 6 Ricci sums
-  // and 22 advection sums per interior vertex
+  // the share of a block that the interface states
   const size_t per_block = sizeof(double) * (kSdComponents * (size_t)g.nvol + 28 * (size_t)npts);
   const size_t room = kScratchBytes - kFdBytes;
   if (per_block > room) {

@@ -51,10 +51,6 @@ __device__ __forceinline__ double fd_d2(const double* __restrict__ f,
 __device__ __forceinline__ double ldo(const double* base, unsigned pb) {
   return __ldg(reinterpret_cast<const double*>(reinterpret_cast<const char*>(base) + pb));
 }
-// The same for memory that the kernel also writes.
-__device__ __forceinline__ double ldm(const double* base, unsigned pb) {
-  return *reinterpret_cast<const double*>(reinterpret_cast<const char*>(base) + pb);
-}
 __device__ __forceinline__ void sto(double* base, unsigned pb, double v) {
   *reinterpret_cast<double*>(reinterpret_cast<char*>(base) + pb) = v;
 }

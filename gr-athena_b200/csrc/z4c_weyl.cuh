@@ -283,21 +283,4 @@ __device__ __forceinline__ void weyl_contract(const double gph[6], const double 
 #undef GUU
 }
 
-// Both phases at one interior vertex.
-__device__ __forceinline__ void weyl_point(const double* __restrict__ uB,
-                                           const double* __restrict__ admB,
-                                           const double* __restrict__ sdB, int64_t nvol,
-                                           int64_t p, const int64_t s[3], const DevParams& P,
-                                           const FdScale& F, double x1, double x2, double x3,
-                                           double* rpsi4, double* ipsi4) {
-  double Rd[6], R, K, DK[3][6], gph[6], Kd[6];
-  weyl_curvature(uB, admB, sdB, nvol, p, s, P, F, Rd, R, K, DK);
-#pragma unroll
-  for (int q = 0; q < 6; ++q) {
-    gph[q] = __ldg(admB + p + (int64_t)(Z4C_ADM_GXX + q) * nvol);
-    Kd[q] = __ldg(admB + p + (int64_t)(Z4C_ADM_KXX + q) * nvol);
-  }
-  weyl_contract(gph, Kd, Rd, R, K, DK, x1, x2, x3, rpsi4, ipsi4);
-}
-
 }  // namespace z4c

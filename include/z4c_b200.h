@@ -593,7 +593,7 @@ int z4c_adj_snapshots(z4c_ctx *ctx, int nsteps, int *nsnap);
  * must not allocate, e.g. at start-up; every later call on that device
  * allocates nothing.  A CUDA error left pending by earlier work is reported
  * (Z4C_ECUDA) before anything is enqueued, not taken for this call's.  Blocks are
- * processed in chunks that fit the array; a MeshBlock whose scratch alone
+ * processed in chunks that fit the array; a MeshBlock whose share alone
  * (33 doubles per vertex, ghosts included, plus 28 per interior vertex)
  * exceeds it -- above roughly 45^3 cells -- is rejected with Z4C_EINVAL
  * before any work is enqueued.  Every call shares

@@ -11,9 +11,9 @@ fit it.
 
 The GPU test compares it with the context-based z4c_rhs on two calls in a row
 (the second on a different state, so that the array's leftover contents from
-the first call would show), on MeshBlocks of 40^3 cells, one per chunk, and on
-64 MeshBlocks of 16^3 cells, whose kernels are the compile-time-geometry
-instances, a dozen blocks per chunk.  Around the second call the device's free
+the first call would show), on MeshBlocks of 40^3 cells, one per chunk in two slabs
+of planes, and on 64 MeshBlocks of 16^3 cells, whose Kreiss-Oliger kernel is the
+compile-time-geometry instance, a dozen blocks per chunk.  Around the second call the device's free
 memory is read: the call must not change it.  The file is named to be
 collected last.
 """
@@ -49,12 +49,11 @@ def test_rejects_bad_sizes_before_any_work():
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("nb,nx", [
-    # 8 blocks of 40^3 cells: 46.5 MB of scratch per block (33 doubles per
-    # vertex, 28 per interior vertex), so the 64 MiB array takes one block
-    # per chunk
+    # 8 blocks of 40^3 cells: 46.5 MB per block by the stated rule (33 doubles
+    # per vertex, 28 per interior vertex), so one block per chunk, and 75 MB of
+    # components, so two slabs of planes in the 64 MiB array
     ((2, 2, 2), 40),
-    # 64 blocks of 16^3 cells (5.2 MB each, 12 per chunk): the fixed-geometry
-    # kernel instances
+    # 64 blocks of 16^3 cells (5.2 MB each, 12 per chunk, whole)
     ((4, 4, 4), 16)])
 def test_noalloc_rhs_matches_context_rhs_on_two_calls(nb, nx):
     from z4c_b200 import initial_data as ID
