@@ -242,7 +242,9 @@ def reference_binary():
     else:
         note = "portable build (-O3 -march=x86-64-v3): no native build present"
     exe = os.path.join(ref, "athena_ref")
-    return (exe if os.path.exists(exe) else None), note
+    if not os.path.exists(exe):
+        return None, "oracle/_ref holds none, and its sources are not on this machine"
+    return exe, note
 
 
 def run_reference_cpu(nlim, threads):
@@ -1146,19 +1148,18 @@ def main_reference(args, rank, world):
     threads = os.cpu_count() or 1
     nlim = max(1, args.steps)
     v, build = run_reference_cpu(nlim, threads)
-    kind = "reference"
-    sample = f"reference OpenMP build, full workload, {nlim} RK4 steps; {build}"
     if v is None:
-        v, n = run_oracle_cpu()
-        kind, threads = "port", 1
-        sample = f"C oracle RHS on {n} MeshBlocks of 16^3, single thread"
+        print(json.dumps({"impl": "reference",
+                          "unavailable": "no reference build to run: " + str(build)}), flush=True)
+        return
+    sample = f"reference OpenMP build, full workload, {nlim} RK4 steps; {build}"
     line = {"metric": METRIC, "value": v, "unit": "zone-updates/s", "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None, "dtype": "f64",
             "data": "synthetic (analytic puncture initial data)",
             "config": dict(WORKLOAD, parallelism="cpu"), "impl": "reference",
             "cpu_baseline": {"value": v, "unit": "zone-updates/s", "cores": threads,
-                             "kind": kind, "sample": sample},
+                             "kind": "reference", "sample": sample},
             "e2e": {"value": v, "unit": "zone-updates/s", "h2d_bytes_per_step": 0,
                     "d2h_bytes_per_step": 0}}
     print(json.dumps(line), flush=True)
