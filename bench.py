@@ -87,8 +87,8 @@ STAGE_BYTES_PER_POINT = 4 * 22 * 8
 # for the low-storage stage update (7 per variable).
 FP64_OPS_PER_POINT_STAGE = 7697 + 154
 # The launches of one fused stage and their measured DRAM traffic per interior
-# vertex (ncu dram__bytes_read.sum + dram__bytes_write.sum summed over them on
-# the 512 blocks; not captured for the merged grid's stage).
+# vertex (ncu dram__bytes_read.sum + dram__bytes_write.sum summed over them, on
+# 128 blocks of 16^3 and on one block of 128^3: profiles/stage_passes.md).
 STAGE_KERNELS = {0: "k_deriv, k_point, k_ko_stage_ls",
                  1: "k_deriv, k_point_fast; on the 128^3 merged grid k_prep, "
                     "k_stencil_point, k_col_fast"}
@@ -98,7 +98,8 @@ FP64_OPS_PER_POINT_WEYL = 7409
 # psi4 extraction spheres of the diagnostics: (radius, nlev, lmax) inside
 # the [-16,16]^3 domain
 WAVE_SPHERES = ((6.0, 30, 8), (12.0, 30, 8))
-STAGE_TRAFFIC_PER_POINT = {0: 11764.0e6 / (512 * 17 ** 3), 1: 9193.0e6 / (512 * 17 ** 3)}
+STAGE_TRAFFIC_PER_POINT = {0: 2894.0e6 / (128 * 17 ** 3), 1: 2266.9e6 / (128 * 17 ** 3),
+                           "merged": 4469.2e6 / 129 ** 3}
 
 
 def parse():
@@ -115,8 +116,8 @@ def parse():
     ap.add_argument("--no-amr", action="store_true",
                     help="skip the adaptive binary-puncture run of the headline line")
     ap.add_argument("--contract", type=int, default=1, choices=[0, 1],
-                    help="1: the contracted path (fused multiply-adds, four launches per "
-                         "stage; the headline); 0: the exact path, bit for bit the "
+                    help="1: the contracted path (fused multiply-adds, two launches per "
+                         "stage, three on the 128^3 merged grid; the headline); 0: the exact path, bit for bit the "
                          "reference's arithmetic (also measured in the headline line)")
     ap.add_argument("--nb", type=int, default=8,
                     help="MeshBlocks per axis (8 = the 128^3 workload; smaller for profiling)")
@@ -1058,7 +1059,9 @@ def main():
     achieved_gbs = STAGE_BYTES_PER_POINT * stage_npts / stage_s / 1e9
     achieved_tf = FP64_OPS_PER_POINT_STAGE * stage_npts / stage_s / 1e12
     path_key = "merged" if merged else args.contract
-    traffic = STAGE_TRAFFIC_PER_POINT.get(path_key)
+    traffic = STAGE_TRAFFIC_PER_POINT[path_key]
+    if merged and args.nb != 8:
+        traffic = None  # measured on the 128^3 grid's passes
     roof = {"bound": "fp64", "achieved": achieved_tf, "peak": fp64_peak_tf, "unit": "TFLOP/s",
             "frac": achieved_tf / fp64_peak_tf,
             "peak_source": "measured in this run: dependent DFMA chains on every SM "

@@ -125,11 +125,11 @@ __device__ __forceinline__ double fd_lx_reg(const double* w, double vx, double l
 // The cost does not depend on the block's size, as the strides of the tile
 // are constants whatever those of the array.
 // Bound by shared-memory reads (its data pipe at 73% of its peak) at 14 warps
-// per SM: 512 blocks of 16^3, 1.19 ms, 4.05 GB of DRAM traffic (3.4 TB/s).  Together with the
-// pointwise pass (0.78 ms, 5.2 TB/s) it replaces stored first derivatives
-// (0.50 ms), Ricci (0.64), advection (0.59) and main (0.72) passes whose
-// stencils went to L1 and L2 at eight warps per SM.  Measured and slower: a
-// column per thread (1.45 ms), separate launches for the variables with and
+// per SM: 512 blocks of 16^3, 1.19 ms, 4.05 GB of DRAM traffic (3.4 TB/s).
+// Together with the pointwise pass (0.78 ms, 5.2 TB/s) it replaces stored first
+// derivatives (0.50 ms), Ricci (0.64), advection (0.59) and main (0.72) passes
+// whose stencils went to L1 and L2 at eight warps per SM.  Measured and slower:
+// a column per thread (1.45 ms), separate launches for the variables with and
 // without second derivatives (0.87 + 0.41), the y stencils moved into the
 // pass that fills D_y (0.87 against 0.79 for the former), and on the
 // contracted path D_z of D_x and D_y from register windows (1.79).
