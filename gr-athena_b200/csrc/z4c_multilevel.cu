@@ -49,6 +49,7 @@ namespace z4c {
 using refine::RefGeom;
 constexpr int kMlNcg = Z4C_NCG;
 constexpr int kMlUnpackThreads = 512;
+constexpr int kMlBatch = 11;  // variables that the gather of a whole state takes at a time
 
 namespace {
 
@@ -86,15 +87,19 @@ __device__ __forceinline__ int ml_zone(int i, int vs, int ve) {
 // coarse buffer (1).  The vertex's zone, multiplicity and contribution range
 // are found once and serve all nvar variables, whose loads are independent
 // of one another; the threads of a warp take consecutive vertices.
-// kMlBatch variables at a time: a contribution's address is formed once for
-// them and their loads are in flight together (a variable at a time with 512
-// threads: 1.67 ms a fill on 512 blocks of 16^3, now 1.17, 4.0 GB).  grid z
-// cuts the vertices so that the last wave is short.
-constexpr int kMlBatch = 11, kMlGatherThreads = 256, kMlGatherParts = 4;
-__global__ void __launch_bounds__(kMlGatherThreads)
+// BATCH variables at a time: a contribution's address is formed once for them
+// and their loads are in flight together.  parts: CTAs that share an array's
+// vertices, neighbours in the grid, so that the lists are read again from L2.
+// A whole fill, us, with a variable at a time | 4 CTAs of 256 threads far apart
+// in the grid | as it is: 64 blocks of 16^3 736 | 259 | 227, 512 blocks 2714 |
+// 2209 | 2077, 3,424 blocks 13830 | 14440 | 11190; two variables (the Weyl
+// scalar) on 3,424 blocks 1643 | 3325, eleven slots for two | 1626.
+template <int BATCH>
+__global__ void __launch_bounds__(kMlUnpackThreads)
 k_ml_unpack(MlPlan P, const double* __restrict__ src, double* __restrict__ dst, int nvar,
-            int reg_nvar) {
-  const int b = blockIdx.x, arr = blockIdx.y;  // arr: 0 fine, 1 coarse
+            int reg_nvar, int parts) {
+  const int b = blockIdx.x / parts, part = blockIdx.x % parts;
+  const int arr = blockIdx.y;  // 0 fine, 1 coarse
   // a coarse buffer that no prolongation reads is not filled
   if (arr == 1 && !P.coarser[b]) return;
   __shared__ unsigned char mult[343];
@@ -116,7 +121,7 @@ k_ml_unpack(MlPlan P, const double* __restrict__ src, double* __restrict__ dst, 
   const int64_t vs = vol;
   const double* own = arr ? P.csrc + (int64_t)b * Z4C_NVAR * vol : src + (int64_t)b * reg_nvar * vol;
   double* out = arr ? P.coarse + (int64_t)b * Z4C_NVAR * vol : dst + (int64_t)b * reg_nvar * vol;
-  for (int p = blockIdx.z * blockDim.x + threadIdx.x; p < vol; p += gridDim.z * blockDim.x) {
+  for (int p = part * blockDim.x + threadIdx.x; p < vol; p += parts * blockDim.x) {
     const int i = p % d0, row = p / d0, j = row % d1, k = row / d1;
     const int zi = ml_zone(i, ng, v0), zj = ml_zone(j, ng, v1), zk = ml_zone(k, ng, v2);
     const int z = (zk * 7 + zj) * 7 + zi;
@@ -124,11 +129,11 @@ k_ml_unpack(MlPlan P, const double* __restrict__ src, double* __restrict__ dst, 
     const int qb = zs[z] - c0, qe = zs[z + 1] - c0;
     const int m = mult[z];
     const double inv = m > 1 ? P.inv[m] : 1.0;
-    for (int n0 = 0; n0 < nvar; n0 += kMlBatch) {
+    for (int n0 = 0; n0 < nvar; n0 += BATCH) {
       const int nn = nvar - n0;
-      double v[kMlBatch];
+      double v[BATCH];
 #pragma unroll
-      for (int n = 0; n < kMlBatch; ++n) v[n] = in && n < nn ? __ldg(own + (n0 + n) * vs + p) : 0.0;
+      for (int n = 0; n < BATCH; ++n) v[n] = in && n < nn ? __ldg(own + (n0 + n) * vs + p) : 0.0;
       for (int q = qb; q < qe; ++q) {
         const MlContrib c = sc[q];
         const int64_t sv = c.scoarse ? P.cvol : P.fvol;
@@ -136,14 +141,14 @@ k_ml_unpack(MlPlan P, const double* __restrict__ src, double* __restrict__ dst, 
         const double* s = (c.scoarse ? P.csrc + ((int64_t)c.sblk * Z4C_NVAR + n0) * sv
                                      : src + ((int64_t)c.sblk * reg_nvar + n0) * sv) +
                           ((k + c.d[2]) * s1 + j + c.d[1]) * s0 + i + c.d[0];
-        double x[kMlBatch];
+        double x[BATCH];
 #pragma unroll
-        for (int n = 0; n < kMlBatch; ++n) x[n] = n < nn ? __ldg(s + n * sv) : 0.0;
+        for (int n = 0; n < BATCH; ++n) x[n] = n < nn ? __ldg(s + n * sv) : 0.0;
 #pragma unroll
-        for (int n = 0; n < kMlBatch; ++n) v[n] = c.mode == kMlCopy ? x[n] : v[n] + x[n];
+        for (int n = 0; n < BATCH; ++n) v[n] = c.mode == kMlCopy ? x[n] : v[n] + x[n];
       }
 #pragma unroll
-      for (int n = 0; n < kMlBatch; ++n)
+      for (int n = 0; n < BATCH; ++n)
         if (n < nn) out[(n0 + n) * vs + p] = m > 1 ? v[n] * inv : v[n];
     }
   }
@@ -975,7 +980,8 @@ int ml_prefer_l1() {  // a hint, given once per device
     if (e == cudaSuccess) e = r;
   };
   prefer((const void*)k_ml_restrict, cudaSharedmemCarveoutMaxL1);
-  prefer((const void*)k_ml_unpack, 25);  // its tables and lists, a few kB per CTA
+  prefer((const void*)k_ml_unpack<2>, 25);  // its tables and lists, a few kB per CTA
+  prefer((const void*)k_ml_unpack<kMlBatch>, 25);
   prefer((const void*)k_ml_prolong, cudaSharedmemCarveoutMaxL1);
   if (e == cudaSuccess) given.fetch_or(bit);
   return (int)e;
@@ -993,12 +999,16 @@ int launch_ml_exchange(const MlPlan& P, const double* src, double* dst, int nvar
     ++launches;
   }
   const size_t smem = sizeof(MlContrib) * (size_t)std::max(P.max_block_contrib, 1);
+  auto unpack = nvar <= 2 ? k_ml_unpack<2> : k_ml_unpack<kMlBatch>;
   if (smem > 48 * 1024 &&
-      cudaFuncSetAttribute(k_ml_unpack, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem) != cudaSuccess)
+      cudaFuncSetAttribute(unpack, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+          cudaSuccess)
     return set_error(Z4C_ECUDA, "multilevel exchange: shared memory for the contribution lists");
-  k_ml_unpack<<<dim3(P.nblocks, 2, kMlGatherParts), kMlGatherThreads, smem, st>>>(
-      P, src, dst, nvar, reg_nvar);
+  // two CTAs per array where the fine arrays alone leave SMs without one (120
+  // blocks of 24^3: 951 us a fill against 1031; 400 of 8^3: 752 against 716)
+  const int parts = P.nblocks < 148 ? 2 : 1;
+  unpack<<<dim3(P.nblocks * parts, 2), kMlUnpackThreads, smem, st>>>(P, src, dst, nvar, reg_nvar,
+                                                                    parts);
   ++launches;
   auto bc_axis = [&](int lv, double* arr, int64_t bstride, int64_t vol, const int* dims, int ng) {
     for (int a = 0; a < 3; ++a) {

@@ -158,6 +158,33 @@ def test_exchange_matches_reference_and_oracle(bc):
     ctx.close()
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("root,nx,levels", [
+    (2, (8, 8, 8), 2),      # 120 blocks: two CTAs share a block's vertices
+    (2, (12, 8, 10), 1),
+    (4, (8, 8, 8), 2),      # 232 blocks: one CTA each
+])
+def test_exchange_of_states_and_of_the_weyl_scalar(root, nx, levels):
+    """The 22 variables of a state and the two of the Weyl scalar, below and
+    above the block count where the gather changes its launch."""
+    half = 16.0
+    boxes = [{**{f"x{a}min": -half / 2 ** lev for a in (1, 2, 3)},
+              **{f"x{a}max": half / 2 ** lev for a in (1, 2, 3)}, "level": lev}
+             for lev in range(1, levels + 1)]
+    mesh = Z.Mesh((root,) * 3, nx, (-half,) * 3, (half,) * 3, "outflow", refinement=boxes)
+    assert (mesh.nblocks < 148) == (root == 2), mesh.nblocks
+    rng = np.random.default_rng(3)
+    ctx = Z.Z4c(mesh, Z.default_params(), "rk4")
+    for reg in (Z.REG_U, Z.REG_WEYL):
+        u = rng.uniform(-1, 1, ctx.shape(reg))
+        ctx.upload(reg, u)
+        ctx.ghost_fill(reg)
+        got = ctx.download(reg)
+        assert bitwise(got, O.ml_exchange(mesh.nb, mesh.root_level, mesh.nx, mesh.bc,
+                                          mesh.locs, u)), reg
+    ctx.close()
+
+
 def sommerfeld_faces(mesh, b):
     """gr_sommerfeld faces of block b of a refined mesh, from its logical
     location at its level."""
