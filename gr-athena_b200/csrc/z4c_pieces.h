@@ -40,19 +40,17 @@ inline DvShares dv_least_shares(int64_t parts, int64_t plane, int nc) {
   return {(parts + kDvGroup - 1) / kDvGroup * kDvGroup, dv_doubles(plane + kDvGroup, nc)};
 }
 // What serves the passes best: every component of the right-hand side (whole)
-// where that is at most a little more, or small on the mesh (512 Mi doubles);
-// every one of the constraints', but no more than 1 GiB on the mesh (512 blocks
-// of 16^3 run as two groups then, at the same time as at once).  The passes
-// run in pieces that fit.
+// where that is at most a little more, or small on the mesh (512 Mi doubles),
+// and every one of the constraints' (an eighth of a 16^3 block's memory; with a
+// seventh of it, two planes, the constraints of one block take 182 us instead
+// of 30).  The passes run in pieces that fit.
 inline DvShares dv_best_shares(const DvShares& least, int64_t whole, int64_t npts, int nc,
                                int nblocks) {
   DvShares s = least;
   if (whole > s.rhs &&
       (whole <= s.rhs + s.rhs / 16 || whole * nblocks <= (int64_t)1 << 29))
     s.rhs = whole;
-  const int64_t con = dv_doubles(npts, nc), cap = dv_share((int64_t)1 << 27, nblocks);
-  if (con <= cap) s.con = con;
-  else if (cap > s.con) s.con = cap;
+  s.con = dv_doubles(npts, nc);
   return s;
 }
 // Allocates the scratch of nblocks blocks: the best shares, or, where the

@@ -1,8 +1,9 @@
 """The derivative pass in pieces, where its scratch does not hold every block
 (csrc/z4c_pieces.h): the same fields as one block of 160^3, whose planes run in
 slabs, as eight blocks of 80^3, which run in two groups, and as single blocks of
-80^3, whole.  A vertex's right-hand side, stage output and constraints depend on
-its own stencils only, so every decomposition gives the same values."""
+80^3, whole; and the constraints of a context that found the device full.  A
+vertex's right-hand side, stage output and constraints depend on its own
+stencils only, so every decomposition gives the same values."""
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -55,13 +56,16 @@ def interior(f):
 POSITIONS = [(i, j, k) for k in range(2) for j in range(2) for i in range(2)]  # block order
 
 
-def outputs(nb, nx, u, contract, integ):
+def outputs(nb, nx, u, contract, integ, full=False):
     """Registers after a right-hand side, a stage and the constraints of u
     [block][22][k][j][i], and the kernels launched by the first and the last."""
     import torch
     import z4c_b200 as Z
     mesh = Z.Mesh((nb,) * 3, (nx,) * 3, (0.0,) * 3, (nb * nx * H,) * 3, "outflow")
+    taken = fill_device(nb ** 3, nx) if full else None
     ctx = Z.Z4c(mesh, Z.default_params(**PUNC), integ)
+    del taken
+    torch.cuda.empty_cache()
     ctx.set_contract(contract)
     view(ctx, Z.REG_U).copy_(u)
     if integ == "rk4":
@@ -88,6 +92,32 @@ def outputs(nb, nx, u, contract, integ):
     return out, (n1 - n0, n2 - n1)
 
 
+def fill_device(nblocks, nx):
+    """Takes the device's memory but for what a low-storage context of nx^3 blocks
+    needs beside its constraints' scratch, and half of that."""
+    import torch
+    nvol, npts = (nx + 9) ** 3, (nx + 1) ** 3
+    # u, w, rhs, u1, adm, con, weyl and the inverse metric; derivatives, Ricci
+    # and advection parts of the scratch, then half of the constraints' 63
+    need = 8 * nblocks * ((4 * 22 + 17 + 7 + 2 + 6 + 33) * nvol + (28 + 63 // 2) * npts)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    free = torch.cuda.mem_get_info()[0]
+    return torch.empty(free - need - (64 << 20), dtype=torch.uint8, device="cuda")
+
+
+def test_context_on_a_full_device_runs_in_smaller_pieces():
+    """Where the preferred scratch is not to be had the context takes the least:
+    the constraints plane by plane, with the same values."""
+    import torch
+    u = fields()
+    best, n = outputs(1, 2 * N, u[None], False, "rk4")
+    least, m = outputs(1, 2 * N, u[None], False, "rk4", full=True)
+    assert n[0] == 2 and m[0] == 2 * (2 * N + 1)
+    for a, b in zip(best, least):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("contract,integ", [(False, "rk4"), (True, "rk4"), (False, "bt_rk4")])
 def test_pieces_give_the_whole_blocks_values(contract, integ):
     import torch
@@ -96,7 +126,7 @@ def test_pieces_give_the_whole_blocks_values(contract, integ):
     groups, ng = outputs(2, N, torch.stack([block(u, p) for p in POSITIONS]), contract, integ)
     # right-hand side: two launches per piece, and Kreiss-Oliger on the exact path
     ko = 0 if contract else 1
-    assert ns == (2 * 2, 2 * 3 + ko) and ng == (2 * 2, 2 * 2 + ko)
+    assert ns == (2, 2 * 3 + ko) and ng == (2, 2 * 2 + ko)
     for b, (i, j, k) in enumerate(POSITIONS):
         whole, nw = outputs(1, N, block(u, (i, j, k))[None], contract, integ)
         assert nw == (2, 2 + ko)

@@ -106,7 +106,7 @@ def test_context_shares(pc, nx):
         assert parts <= least[0] <= parts + 31
         assert least[0] <= best[0] and least[1] <= best[1]
         assert best[0] <= max(least[0] + least[0] // 16, 2 ** 29 // nblocks)
-        assert best[1] <= max(least[1], 2 ** 27 // nblocks)
+        assert best[1] == pc.pc_doubles(LL((nx[0] + 1) * (nx[1] + 1) * (nx[2] + 1)), CON)
         for s in (least, best):
             assert s[0] % 32 == 0 and s[1] % 32 == 0
             for comps, share in ((COMPONENTS, s[0]), (CON, s[1])):
