@@ -50,6 +50,8 @@ using refine::RefGeom;
 constexpr int kMlNcg = Z4C_NCG;
 constexpr int kMlUnpackThreads = 512;
 constexpr int kMlBatch = 11;  // variables that the gather of a whole state takes at a time
+// Threads of the gather's CTAs: two CTAs of either fit an SM's registers.
+constexpr int ml_gather_threads(int batch) { return batch == kMlBatch ? 384 : 512; }
 
 namespace {
 
@@ -91,11 +93,13 @@ __device__ __forceinline__ int ml_zone(int i, int vs, int ve) {
 // and their loads are in flight together.  parts: CTAs that share an array's
 // vertices, neighbours in the grid, so that the lists are read again from L2.
 // A whole fill, us, with a variable at a time | 4 CTAs of 256 threads far apart
-// in the grid | as it is: 64 blocks of 16^3 736 | 259 | 227, 512 blocks 2714 |
-// 2209 | 2077, 3,424 blocks 13830 | 14440 | 11190; two variables (the Weyl
-// scalar) on 3,424 blocks 1643 | 3325, eleven slots for two | 1626.
+// in the grid | as it is: 64 blocks of 16^3 736 | 259 | 209, 512 blocks 2714 |
+// 2209 | 1739, 3,424 blocks 13830 | 14440 | 8870; two variables (the Weyl
+// scalar) on 3,424 blocks 1643 | 3325, eleven slots for two | 1635.  With 512
+// threads for eleven variables 228, 2089 and 11260 (one CTA per SM), or with
+// its registers cut to 64 for two of them 223, 1876 and 9760.
 template <int BATCH>
-__global__ void __launch_bounds__(kMlUnpackThreads)
+__global__ void __launch_bounds__(ml_gather_threads(BATCH), 2)
 k_ml_unpack(MlPlan P, const double* __restrict__ src, double* __restrict__ dst, int nvar,
             int reg_nvar, int parts) {
   const int b = blockIdx.x / parts, part = blockIdx.x % parts;
@@ -999,16 +1003,18 @@ int launch_ml_exchange(const MlPlan& P, const double* src, double* dst, int nvar
     ++launches;
   }
   const size_t smem = sizeof(MlContrib) * (size_t)std::max(P.max_block_contrib, 1);
-  auto unpack = nvar <= 2 ? k_ml_unpack<2> : k_ml_unpack<kMlBatch>;
+  const bool few = nvar <= 2;
+  auto unpack = few ? k_ml_unpack<2> : k_ml_unpack<kMlBatch>;
   if (smem > 48 * 1024 &&
       cudaFuncSetAttribute(unpack, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
           cudaSuccess)
     return set_error(Z4C_ECUDA, "multilevel exchange: shared memory for the contribution lists");
-  // two CTAs per array where the fine arrays alone leave SMs without one (120
-  // blocks of 24^3: 951 us a fill against 1031; 400 of 8^3: 752 against 716)
-  const int parts = P.nblocks < 148 ? 2 : 1;
-  unpack<<<dim3(P.nblocks * parts, 2), kMlUnpackThreads, smem, st>>>(P, src, dst, nvar, reg_nvar,
-                                                                    parts);
+  // two CTAs per array; for two variables only where the fine arrays alone leave
+  // SMs without one (64 blocks: 94 us a fill against 116; 3,424: 1692 against
+  // 1635, for a state 8872 against 9856)
+  const int parts = few && P.nblocks >= 148 ? 1 : 2;
+  unpack<<<dim3(P.nblocks * parts, 2), ml_gather_threads(few ? 2 : kMlBatch), smem, st>>>(
+      P, src, dst, nvar, reg_nvar, parts);
   ++launches;
   auto bc_axis = [&](int lv, double* arr, int64_t bstride, int64_t vol, const int* dims, int ng) {
     for (int a = 0; a < 3; ++a) {

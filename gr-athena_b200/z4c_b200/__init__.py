@@ -675,7 +675,7 @@ class Z4c:
         _check(lib().z4c_set_contract(self._h, int(bool(on))))
 
     def set_point_regs(self, regs):
-        """Register budget of the heavy RHS passes (0 or 168, see
+        """Kept for callers, selects nothing (0 or 168, see
         z4c_set_point_regs)."""
         _check(lib().z4c_set_point_regs(self._h, int(regs)))
 

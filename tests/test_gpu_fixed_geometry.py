@@ -1,8 +1,8 @@
 """The compile-time 16^3 kernel instances against the oracle.
 
-The golden fixtures use 8^3 MeshBlocks, which run the generic kernels; every
-kernel of the step also exists in a form specialised for 16^3 MeshBlocks
-(constant strides, whole-loop unrolling).  Here meshes of 2^3 and 3^3
+The golden fixtures use 8^3 MeshBlocks, which run the generic kernels; the
+stage, exchange, boundary and AlgConstr kernels also exist in a form specialised
+for 16^3 MeshBlocks (constant strides, whole-loop unrolling).  Here meshes of 2^3 and 3^3
 MeshBlocks of 16^3 take one full step through the captured graph for each
 integrator and boundary condition, including the Sommerfeld and Butcher
 stage kernels, and are compared with the same step on the oracle."""

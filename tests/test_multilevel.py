@@ -162,7 +162,7 @@ def test_exchange_matches_reference_and_oracle(bc):
 @pytest.mark.parametrize("root,nx,levels", [
     (2, (8, 8, 8), 2),      # 120 blocks: two CTAs share a block's vertices
     (2, (12, 8, 10), 1),
-    (4, (8, 8, 8), 2),      # 232 blocks: one CTA each
+    (4, (8, 8, 8), 2),      # 176 blocks: one CTA each for the Weyl scalar
 ])
 def test_exchange_of_states_and_of_the_weyl_scalar(root, nx, levels):
     """The 22 variables of a state and the two of the Weyl scalar, below and
