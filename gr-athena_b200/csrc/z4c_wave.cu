@@ -305,7 +305,9 @@ __global__ void k_wave_project(const double* __restrict__ data, const double* __
   double pr = 0.0, pi = 0.0;
   if (mpl <= 2 * l) {
     const double* Y = ylm + (int64_t)slot * npts * 2;
-    for (int p = seg[sg]; p < seg[sg + 1]; ++p) {
+    const int end = seg[sg + 1];
+#pragma unroll 2  // two vertices' loads in flight; the sums stay in order
+    for (int p = seg[sg]; p < end; ++p) {
       const double dr = data[p], di = data[npts + p];
       const double wt = pw[2 * p], bz = pw[2 * p + 1];
       const double yr = Y[2 * p], yi = Y[2 * p + 1];
@@ -467,10 +469,13 @@ void launch_wave(const Grid& g, const WaveSphere& w, const double* weyl, cudaStr
     k_wave_interp<<<w.npts, 2 * kSten * kSten, 0, st>>>(g, weyl, w.blk, w.base, w.coef, w.data,
                                                        w.npts);
     const int nt = w.nseg * w.nslot;
-    // 128 threads: the warps of a CTA find the vertices' values in its L1 (9,002
-    // vertices: 473 us, against 489 with 32 threads and eight loads in flight)
-    k_wave_project<<<(nt + 127) / 128, 128, 0, st>>>(w.data, w.pw, w.ylm, w.seg, w.loc, w.npts,
-                                                     w.nseg, w.nslot, w.lmax);
+    // 64 threads, two vertices at a time: a sphere of 9,002 vertices on 1 | 64
+    // blocks of 16^3, psi4 and its extraction, 1271 | 942 us, against 1365 | 987
+    // with 32 threads and eight at a time (fewer warps find the vertices' values
+    // in an L1) and 1636 | 974 with 128 threads and the compiler's unrolling;
+    // 362 vertices on 3 blocks 150, 154 and 166
+    k_wave_project<<<(nt + 63) / 64, 64, 0, st>>>(w.data, w.pw, w.ylm, w.seg, w.loc, w.npts,
+                                                  w.nseg, w.nslot, w.lmax);
     add_kernel_launches(2);
   }
   k_wave_reduce<<<(2 * w.nslot + 127) / 128, 128, 0, st>>>(w.loc, w.psi, w.nseg, w.nslot);
